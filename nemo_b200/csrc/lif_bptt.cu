@@ -219,13 +219,12 @@ k_back(Net n, int t, const float* wOut, const float* uSeg, int segStart, const f
 	}
 }
 
-/* dL/dw over one segment: for every in-synapse k of neuron i, the sum over
- * the segment's steps and the trials of gu[t]_i * x_k[t]; warp per neuron,
- * lanes summing their trial over the steps, one reduction per synapse. */
-template<bool RELAXED>
+/* dL/dw over one segment of the relaxed model: for every in-synapse k of
+ * neuron i, the sum over the segment's steps and the trials of gu[t]_i *
+ * x_k[t]; warp per neuron, lanes summing their trial over the steps, one
+ * reduction per synapse. */
 __global__ void __launch_bounds__(THREADS)
-k_dw(Net n, int segStart, int segEnd, const float* guSeg, const uint32_t* sBits, const float* sF,
-		const uint32_t* inBits, float* dw)
+k_dw_relaxed(Net n, int segStart, int segEnd, const float* guSeg, const float* sF, const uint32_t* inBits, float* dw)
 {
 	const uint32_t lane = threadIdx.x & 31u;
 	const int warps = int((gridDim.x * blockDim.x) >> 5);
@@ -235,16 +234,8 @@ k_dw(Net n, int segStart, int segEnd, const float* guSeg, const uint32_t* sBits,
 			const int p = n.pre[k];
 			float acc = 0.0f;
 			for(int t = segStart; t < segEnd; ++t) {
-				if(RELAXED) {
-					const float g = guSeg[(size_t(t - segStart) * n.N + i) * 32 + lane];
-					acc = __fadd_rn(acc, __fmul_rn(g, presyn<RELAXED>(n, p, t, lane, sBits, sF, inBits)));
-				} else {
-					/* spikes are 0 or 1: add gu where the trial's bit is set */
-					const uint32_t word = presynWord(n, p, t, sBits, inBits);
-					if(word && ((word >> lane) & 1u)) {
-						acc = __fadd_rn(acc, guSeg[(size_t(t - segStart) * n.N + i) * 32 + lane]);
-					}
-				}
+				const float g = guSeg[(size_t(t - segStart) * n.N + i) * 32 + lane];
+				acc = __fadd_rn(acc, __fmul_rn(g, presyn<true>(n, p, t, lane, nullptr, sF, inBits)));
 			}
 #pragma unroll
 			for(int d = 16; d; d >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(FULL, acc, d));
@@ -253,60 +244,197 @@ k_dw(Net n, int segStart, int segEnd, const float* guSeg, const uint32_t* sBits,
 	}
 }
 
-/* dL/dw over one segment for spikes as bits: lanes over the neuron's
- * in-synapses, each lane walking its synapse's presynaptic words along the
- * segment (words stored source-major, [unit][T], so consecutive steps are
- * consecutive words) and adding gu[t]_i of every trial whose bit is set. */
+/* ---- event lists (spikes as bits) ----
+ *
+ * The recompute and the weight gradient of a segment both go over every
+ * synapse and every (step, trial) in which its presynaptic unit spikes. The
+ * spikes are known, so each unit's (step, trial) pairs of the segment are
+ * listed once (k_events) and every synapse walks its unit's list: the work is
+ * the number of spikes times the fan-out, where walking words tests every
+ * (step, synapse) word and shuffles every one that is not 0 (a gradient step
+ * of 10,000 neurons, 2.5e6 synapses, 500 steps and 32 trials on a B200: 62.4 ms
+ * with a launch per recomputed step, 48.5 with the lists). A segment is
+ * taken in parts of at most PART_STEPS steps, the most for which a neuron's
+ * currents of all steps and trials stay in shared memory (8 KB a warp) and a
+ * code step * 32 + trial fits 16 bits. */
+
+const int PART_STEPS = 64;
+const int PART_WARPS = 8;
+
+/* parts of a segment of `steps` steps and the steps of each (the last one
+ * may have fewer) */
+static int parts(int steps) { return (steps + PART_STEPS - 1) / PART_STEPS; }
+static int partSteps(int steps) { return (steps + parts(steps) - 1) / parts(steps); }
+
+/* The event lists of the steps [c0, c1): for part y (steps from c0 + y L) and
+ * presynaptic unit p (neurons, then input channels) the codes (t - part
+ * start) * 32 + b of the spikes it delivers, by step, then by trial, in
+ * codes[(y * units + p) * L * 32 ...], their number in cnt[y * units + p]. A
+ * list is filled up to a multiple of 8 codes with the code L * 32 (a cell
+ * that holds 0). A block takes 32 units of one part: their words are read
+ * coalesced over the units and turned in shared memory, a warp then has a
+ * unit's steps in its lanes. */
 __global__ void __launch_bounds__(THREADS)
-k_dw_bits(Net n, int segStart, int segEnd, const float* guSeg, const uint32_t* sT, const uint32_t* inT, float* dw)
+k_events(Net n, int c0, int c1, int L, const uint32_t* sBits, const uint32_t* inBits, uint16_t* codes, uint32_t* cnt)
 {
+	__shared__ uint32_t tile[PART_STEPS][33];
 	const uint32_t lane = threadIdx.x & 31u;
+	const int warp = int(threadIdx.x >> 5);
+	const int units = n.N + n.C;
+	const int unit0 = int(blockIdx.x) * 32;
+	const int t0 = c0 + int(blockIdx.y) * L;
+	const int len = min(L, c1 - t0);
+	const uint32_t trials = n.B == 32 ? FULL : (1u << n.B) - 1u;
+	for(int r = warp; r < len; r += int(THREADS / 32)) {
+		const int p = unit0 + int(lane);
+		tile[r][lane] = p < units ? presynWord(n, p, t0 + r, sBits, inBits) & trials : 0u;
+	}
+	__syncthreads();
+	for(int q = warp; q < 32; q += int(THREADS / 32)) {
+		const int p = unit0 + q;
+		if(p >= units) break;
+		uint16_t* out = codes + (size_t(blockIdx.y) * units + p) * (size_t(L) * 32);
+		uint32_t total = 0;
+		for(int r0 = 0; r0 < len; r0 += 32) {
+			const int r = r0 + int(lane);
+			uint32_t word = r < len ? tile[r][q] : 0u;
+			const uint32_t c = uint32_t(__popc(word));
+			uint32_t incl = c;
+#pragma unroll
+			for(int d = 1; d < 32; d <<= 1) {
+				const uint32_t x = __shfl_up_sync(FULL, incl, d);
+				if(lane >= uint32_t(d)) incl += x;
+			}
+			uint32_t at = total + incl - c;
+			while(word) {
+				out[at++] = uint16_t(r * 32 + __ffs(int(word)) - 1);
+				word &= word - 1u;
+			}
+			total += __shfl_sync(FULL, incl, 31);
+		}
+		const uint32_t fill = (8u - (total & 7u)) & 7u;
+		if(lane < fill) out[total + lane] = uint16_t(L * 32);
+		if(lane == 0) cnt[size_t(blockIdx.y) * units + p] = total;
+	}
+}
+
+/* The steps [t0, t1) (one part) from v before them (vIn): u of every step
+ * into uOut (segment buffer [K][N][32]), v after them into vOut. Warp per
+ * neuron: its currents of all steps and trials are accumulated in shared
+ * memory, synapse after synapse in order, a synapse's events over the lanes
+ * (distinct cells); a cell so gets its weights in synapse order, as in the
+ * forward, and u is bit-identical. The codes of the next synapses are loaded
+ * while the last ones are added. */
+__global__ void __launch_bounds__(PART_WARPS * 32)
+k_recompute(Net n, int t0, int t1, int segStart, int L, const float* w, const uint16_t* codes, const uint32_t* cnt,
+		const float* vIn, float* vOut, float* uOut)
+{
+	extern __shared__ float sCur[];
+	const int U = 4;
+	const uint32_t lane = threadIdx.x & 31u;
+	const bool active = lane < uint32_t(n.B);
+	float* cur = sCur + size_t(threadIdx.x >> 5) * (size_t(L) * 32);
+	const size_t cap = size_t(L) * 32;
+	const int len = t1 - t0;
 	const int warps = int((gridDim.x * blockDim.x) >> 5);
 	for(int i = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n.N; i += warps) {
+		for(int r = 0; r < len; ++r) cur[r * 32 + int(lane)] = 0.0f;
+		__syncwarp();
 		const int k0 = n.rowptr[i], k1 = n.rowptr[i + 1];
 		for(int base = k0; base < k1; base += 32) {
 			const int k = base + int(lane);
-			if(k >= k1) continue;
-			const int p = n.pre[k];
-			const bool input = p >= n.N;
-			const uint32_t* words = input ? inT + size_t(p - n.N) * n.T : sT + size_t(p) * n.T;
-			float acc = 0.0f;
-			for(int t = segStart; t < segEnd; ++t) {
-				uint32_t word = input ? words[t] : (t == 0 ? 0u : words[t - 1]);
-				while(word) {
-					const int b = __ffs(int(word)) - 1;
-					word &= word - 1u;
-					acc = __fadd_rn(acc, __ldg(&guSeg[(size_t(t - segStart) * n.N + i) * 32 + b]));
+			const int p = k < k1 ? n.pre[k] : 0;
+			const float wk = k < k1 ? w[k] : 0.0f;
+			const uint32_t ck = k < k1 ? cnt[p] : 0u;
+			const int nk = min(32, k1 - base);
+			uint32_t next[U];
+#pragma unroll
+			for(int x = 0; x < U; ++x) {
+				const uint32_t c = __shfl_sync(FULL, ck, x);
+				const int pq = __shfl_sync(FULL, p, x);
+				next[x] = lane < c ? codes[size_t(pq) * cap + lane] : 0u;
+			}
+			for(int q0 = 0; q0 < nk; q0 += U) {
+				uint32_t code[U];
+#pragma unroll
+				for(int x = 0; x < U; ++x) {
+					code[x] = next[x];
+					const int q = (q0 + U + x) & 31;
+					const uint32_t c = q0 + U + x < nk ? __shfl_sync(FULL, ck, q) : 0u;
+					const int pq = __shfl_sync(FULL, p, q);
+					next[x] = lane < c ? codes[size_t(pq) * cap + lane] : 0u;
 				}
+#pragma unroll
+				for(int x = 0; x < U; ++x) {
+					/* past the last synapse: a count of 0 */
+					const int q = q0 + x;
+					const uint32_t c = __shfl_sync(FULL, ck, q);
+					const float wq = __shfl_sync(FULL, wk, q);
+					if(lane < c) cur[code[x]] = __fadd_rn(cur[code[x]], wq);
+					if(c > 32u) {
+						const uint16_t* more = codes + size_t(__shfl_sync(FULL, p, q)) * cap;
+						for(uint32_t e = 32u + lane; e < c; e += 32u) cur[more[e]] = __fadd_rn(cur[more[e]], wq);
+					}
+					__syncwarp();
+				}
+			}
+		}
+		const size_t cell = size_t(i) * 32 + lane;
+		float v = vIn[cell];
+		for(int r = 0; r < len; ++r) {
+			const float u = __fadd_rn(__fmul_rn(n.beta, v), cur[r * 32 + int(lane)]);
+			const float s = (active && u >= n.theta) ? 1.0f : 0.0f;
+			v = __fsub_rn(u, __fmul_rn(n.theta, s));
+			uOut[(size_t(t0 - segStart + r) * n.N) * 32 + cell] = u;
+		}
+		vOut[cell] = v;
+		__syncwarp();
+	}
+}
+
+/* dL/dw of the steps [t0, t1) (one part): warp per neuron, its gu of the
+ * part's steps in shared memory, lanes over its in-synapses; each lane sums
+ * gu over its presynaptic unit's events, by step, then by trial, eight codes
+ * a load. */
+__global__ void __launch_bounds__(PART_WARPS * 32)
+k_dw_events(Net n, int t0, int t1, int segStart, int L, const float* guSeg, const uint16_t* codes, const uint32_t* cnt,
+		float* dw)
+{
+	extern __shared__ float sGu[];
+	const uint32_t lane = threadIdx.x & 31u;
+	const size_t cap = size_t(L) * 32;
+	float* g = sGu + size_t(threadIdx.x >> 5) * (cap + 32);
+	const int len = t1 - t0;
+	const int warps = int((gridDim.x * blockDim.x) >> 5);
+	g[cap + lane] = 0.0f;
+	for(int i = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n.N; i += warps) {
+		for(int r = 0; r < len; ++r) {
+			g[r * 32 + int(lane)] = guSeg[(size_t(t0 - segStart + r) * n.N + i) * 32 + lane];
+		}
+		__syncwarp();
+		const int k0 = n.rowptr[i], k1 = n.rowptr[i + 1];
+		for(int k = k0 + int(lane); k < k1; k += 32) {
+			const int p = n.pre[k];
+			const uint32_t c = cnt[p];
+			const uint4* list = reinterpret_cast<const uint4*>(codes + size_t(p) * cap);
+			float acc = 0.0f;
+			uint4 next = c ? list[0] : make_uint4(0u, 0u, 0u, 0u);
+			for(uint32_t e = 0; e < c; e += 8u) {
+				const uint4 x = next;
+				if(e + 8u < c) next = list[(e >> 3) + 1u];
+				acc = __fadd_rn(acc, g[x.x & 0xffffu]);
+				acc = __fadd_rn(acc, g[x.x >> 16]);
+				acc = __fadd_rn(acc, g[x.y & 0xffffu]);
+				acc = __fadd_rn(acc, g[x.y >> 16]);
+				acc = __fadd_rn(acc, g[x.z & 0xffffu]);
+				acc = __fadd_rn(acc, g[x.z >> 16]);
+				acc = __fadd_rn(acc, g[x.w & 0xffffu]);
+				acc = __fadd_rn(acc, g[x.w >> 16]);
 			}
 			dw[k] = __fadd_rn(dw[k], acc);
 		}
+		__syncwarp();
 	}
-}
-
-/* dst[c][r] = src[r][c] for a rows x cols array of words */
-__global__ void
-k_transpose(const uint32_t* src, uint32_t* dst, int rows, int cols)
-{
-	__shared__ uint32_t tile[32][33];
-	const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-	for(int y = threadIdx.y; y < 32; y += blockDim.y) {
-		const int r = r0 + y, c = c0 + int(threadIdx.x);
-		if(r < rows && c < cols) tile[y][threadIdx.x] = src[size_t(r) * cols + c];
-	}
-	__syncthreads();
-	for(int y = threadIdx.y; y < 32; y += blockDim.y) {
-		const int c = c0 + y, r = r0 + int(threadIdx.x);
-		if(r < rows && c < cols) dst[size_t(c) * rows + r] = tile[threadIdx.x][y];
-	}
-}
-
-static void
-transpose(const uint32_t* src, uint32_t* dst, int rows, int cols, cudaStream_t st)
-{
-	if(rows == 0 || cols == 0) return;
-	dim3 g((cols + 31) / 32, (rows + 31) / 32), b(32, 8);
-	k_transpose<<<g, b, 0, st>>>(src, dst, rows, cols);
 }
 
 static int
@@ -344,15 +472,36 @@ validate(const Net& n)
 
 using namespace nemo_b200;
 
-/* work buffer: v state [N][32], gu of the step after the segment [N][32],
- * the segment's u and gu [K][N][32], the spike and input words transposed to
- * [unit][T], then the recurrent weights in out-synapse order [nnzRec] */
-static size_t
-workFloats(const lif::Net& n)
-{
-	return size_t(n.N) * 32 * (2 + 2 * size_t(n.K)) + (size_t(n.N) + size_t(n.C)) * size_t(n.T)
-		+ size_t(n.nnzRec);
-}
+/* The work buffer: v state [N][32], gu of the step after the segment [N][32],
+ * the segment's u and gu [K][N][32], the event lists of its parts (codes, then
+ * counts), then the recurrent weights in out-synapse order [nnzRec]. Made
+ * from the buffer's start rounded up to 128 bytes (the size has the slack). */
+struct LifWork {
+	float *v, *guNext, *uSeg, *guSeg;
+	uint16_t* codes;
+	uint32_t* cnt;
+	float* wOut;
+	size_t bytes;
+
+	LifWork(const lif::Net& n, float* base)
+	{
+		const size_t align = 128;
+		char* p = reinterpret_cast<char*>((reinterpret_cast<size_t>(base) + align - 1) / align * align);
+		char* const p0 = p;
+		auto take = [&](size_t bytes) { char* q = p; p += (bytes + align - 1) / align * align; return q; };
+		const int K = std::min(n.K, n.T);
+		const size_t NS = size_t(n.N) * 32, units = size_t(n.N) + size_t(n.C);
+		v = reinterpret_cast<float*>(take(NS * 4));
+		guNext = reinterpret_cast<float*>(take(NS * 4));
+		uSeg = reinterpret_cast<float*>(take(size_t(K) * NS * 4));
+		guSeg = reinterpret_cast<float*>(take(size_t(K) * NS * 4));
+		const size_t Y = size_t(lif::parts(K));
+		codes = reinterpret_cast<uint16_t*>(take(Y * units * size_t(lif::partSteps(K)) * 32 * 2));
+		cnt = reinterpret_cast<uint32_t*>(take(Y * units * 4));
+		wOut = reinterpret_cast<float*>(take(size_t(n.nnzRec) * 4));
+		bytes = size_t(p - p0) + align;
+	}
+};
 
 static std::string g_lifError;
 
@@ -371,7 +520,8 @@ nemo_b200_lif_work_bytes(const nemo_b200_lif_net* net)
 	lif::Net n;
 	static_assert(sizeof(nemo_b200_lif_net) == sizeof(lif::Net), "layout");
 	memcpy(&n, net, sizeof(n));
-	return workFloats(n) * sizeof(float);
+	/* sizes that the calls refuse (validate) need no buffer */
+	return n.N > 0 && n.T > 0 && n.K > 0 && n.C >= 0 && n.nnzRec >= 0 ? LifWork(n, nullptr).bytes : 0;
 }
 
 int
@@ -383,7 +533,7 @@ nemo_b200_lif_forward(const nemo_b200_lif_net* net, const float* w, const uint32
 		memcpy(&n, net, sizeof(n));
 		lif::validate(n);
 		cudaStream_t st = static_cast<cudaStream_t>(stream);
-		float* v = work;
+		float* v = LifWork(n, work).v;
 		NEMO_CUDA(cudaMemsetAsync(v, 0, size_t(n.N) * 32 * 4, st));
 		NEMO_CUDA(cudaMemsetAsync(counts, 0, size_t(n.B) * (n.T / n.binSteps) * 4, st));
 		const int g = lif::grid(n.N);
@@ -411,46 +561,55 @@ nemo_b200_lif_backward(const nemo_b200_lif_net* net, const float* w, const uint3
 		lif::validate(n);
 		cudaStream_t st = static_cast<cudaStream_t>(stream);
 		const size_t NS = size_t(n.N) * 32;
-		float* v = work;
-		float* guNextSeg = work + NS;          /* gu of the first step after the segment */
-		float* uSeg = work + 2 * NS;
-		float* guSeg = uSeg + size_t(n.K) * NS;
-		uint32_t* sT = reinterpret_cast<uint32_t*>(guSeg + size_t(n.K) * NS);
-		uint32_t* inT = sT + size_t(n.N) * n.T;
-		if(!relaxed) {
-			lif::transpose(s_bits, sT, n.T, n.N, st);
-			lif::transpose(in_bits, inT, n.T, n.C, st);
-		}
+		const LifWork k(n, work);
 		const int g = lif::grid(n.N);
 		/* the recurrent weights in out-synapse order, for k_back */
-		float* wOut = reinterpret_cast<float*>(inT + size_t(n.C) * n.T);
-		if(n.nnzRec) lif::k_gather_out<<<g, lif::THREADS, 0, st>>>(n, n.nnzRec, w, wOut);
+		if(n.nnzRec) lif::k_gather_out<<<g, lif::THREADS, 0, st>>>(n, n.nnzRec, w, k.wOut);
 		const int segments = (n.T + n.K - 1) / n.K;
+		const size_t units = size_t(n.N) + size_t(n.C);
+		const int L = lif::partSteps(std::min(n.K, n.T));
+		const unsigned gp = unsigned((n.N + lif::PART_WARPS - 1) / lif::PART_WARPS);
+		const size_t smemU = size_t(lif::PART_WARPS) * L * 32 * 4, smemW = smemU + lif::PART_WARPS * 32 * 4;
+		if(!relaxed) {
+			NEMO_CUDA(cudaFuncSetAttribute(lif::k_recompute, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemU)));
+			NEMO_CUDA(cudaFuncSetAttribute(lif::k_dw_events, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemW)));
+		}
 		for(int sgi = segments - 1; sgi >= 0; --sgi) {
-			const int c0 = sgi * n.K, c1 = std::min(n.T, c0 + n.K);
+			const int c0 = sgi * n.K, c1 = int(std::min<long>(n.T, long(c0) + n.K));
+			const float* ckpt = v_ckpt + size_t(sgi) * NS;
+			const int Y = (c1 - c0 + L - 1) / L;
 			/* recompute u over the segment from its checkpoint */
-			NEMO_CUDA(cudaMemcpyAsync(v, v_ckpt + size_t(sgi) * NS, NS * 4, cudaMemcpyDeviceToDevice, st));
-			for(int t = c0; t < c1; ++t) {
-				if(relaxed) {
+			if(relaxed) {
+				NEMO_CUDA(cudaMemcpyAsync(k.v, ckpt, NS * 4, cudaMemcpyDeviceToDevice, st));
+				for(int t = c0; t < c1; ++t) {
 					lif::k_step<true, true><<<g, lif::THREADS, 0, st>>>(n, t, w, in_bits, nullptr,
-							const_cast<float*>(s_float), v, nullptr, nullptr, uSeg, c0);
-				} else {
-					lif::k_step<false, true><<<g, lif::THREADS, 0, st>>>(n, t, w, in_bits,
-							const_cast<uint32_t*>(s_bits), nullptr, v, nullptr, nullptr, uSeg, c0);
+							const_cast<float*>(s_float), k.v, nullptr, nullptr, k.uSeg, c0);
+				}
+			} else {
+				lif::k_events<<<dim3(unsigned((units + 31) / 32), unsigned(Y)), lif::THREADS, 0, st>>>(n, c0, c1, L, s_bits,
+						in_bits, k.codes, k.cnt);
+				for(int y = 0; y < Y; ++y) {
+					const int t0 = c0 + y * L, t1 = std::min(c1, t0 + L);
+					lif::k_recompute<<<gp, lif::PART_WARPS * 32, smemU, st>>>(n, t0, t1, c0, L, w,
+							k.codes + size_t(y) * units * L * 32, k.cnt + size_t(y) * units, y ? k.v : ckpt, k.v, k.uSeg);
 				}
 			}
 			/* backwards through the segment */
 			for(int t = c1 - 1; t >= c0; --t) {
 				const bool last = t == n.T - 1;
-				const float* next = t == c1 - 1 ? guNextSeg : guSeg + size_t(t + 1 - c0) * NS;
-				lif::k_back<<<g, lif::THREADS, 0, st>>>(n, t, wOut, uSeg, c0, next, guSeg, dcounts, last);
+				const float* next = t == c1 - 1 ? k.guNext : k.guSeg + size_t(t + 1 - c0) * NS;
+				lif::k_back<<<g, lif::THREADS, 0, st>>>(n, t, k.wOut, k.uSeg, c0, next, k.guSeg, dcounts, last);
 			}
 			if(relaxed) {
-				lif::k_dw<true><<<g, lif::THREADS, 0, st>>>(n, c0, c1, guSeg, s_bits, s_float, in_bits, dw);
+				lif::k_dw_relaxed<<<g, lif::THREADS, 0, st>>>(n, c0, c1, k.guSeg, s_float, in_bits, dw);
 			} else {
-				lif::k_dw_bits<<<g, lif::THREADS, 0, st>>>(n, c0, c1, guSeg, sT, inT, dw);
+				for(int y = 0; y < Y; ++y) {
+					const int t0 = c0 + y * L, t1 = std::min(c1, t0 + L);
+					lif::k_dw_events<<<gp, lif::PART_WARPS * 32, smemW, st>>>(n, t0, t1, c0, L, k.guSeg,
+							k.codes + size_t(y) * units * L * 32, k.cnt + size_t(y) * units, dw);
+				}
 			}
-			NEMO_CUDA(cudaMemcpyAsync(guNextSeg, guSeg, NS * 4, cudaMemcpyDeviceToDevice, st));
+			NEMO_CUDA(cudaMemcpyAsync(k.guNext, k.guSeg, NS * 4, cudaMemcpyDeviceToDevice, st));
 		}
 		NEMO_CUDA(cudaGetLastError());
 	})
