@@ -24,7 +24,8 @@
  *     the inbox of cycle t+1 (global reductions; 5% of the synapses for
  *     delays U{1..20}); overlapped with
  *   - the gather of cycle t-1: every block reads the fired sources of cycle
- *     t-1 (all blocks' lists) and, for each, its segment of region b, adding
+ *     t-1 (the lists of the blocks that have synapses into it) and, for each,
+ *     its segment of region b, adding
  *     each weight of delay d >= 2 into slot (t-1+d) mod Q of the target (E or
  *     I by sign), and the STDP accumulation of cycle t-1 over all blocks'
  *     post-spiking targets, dealt out over the grid as entries of at most
@@ -55,6 +56,10 @@ const uint32_t APPLY_PER_LANE = 4;
 /* forward records a gather lane loads per round (a unit of 32 sources of
  * about 7 records each in a block's region takes one or two rounds) */
 const int GATHER_PER_LANE = 4;
+/* records of an average gather unit: two rounds of a warp's loads. Longer units
+ * (32 sources with buckets of 30 records where a batch's instances stay in a
+ * few blocks) left the phase waiting for one warp */
+const uint32_t GATHER_UNIT = 2 * 32 * GATHER_PER_LANE;
 /* plastic synapses a lane visits in one STDP accumulation entry (an entry is
  * a run of at most STDP_ITEM synapses of one post-spiking target) */
 const uint32_t STDP_PER_LANE = 4;
@@ -110,6 +115,13 @@ struct NetDev {
 	 * srcChunk[(s + 1) * groups + g]) ((nDev + 1) * groups entries, derived
 	 * from segOff by launchSourceChunks) */
 	const uint32_t* srcChunk;
+	/* the blocks with a synapse of delay >= 2 into block b, ascending:
+	 * fromList[fromStart[b] .. fromStart[b + 1]) */
+	const uint32_t* fromStart;     /* [blocks + 1] */
+	const uint32_t* fromList;
+	/* fired sources of a gather unit: 32, 16, 8 or 4, so that a unit of
+	 * average buckets has at most GATHER_UNIT records */
+	uint32_t gatherSources;
 	const uint32_t* outDegree;     /* [nDev] synapses per source */
 	const uint32_t* d1Start;       /* [nDev + 1] */
 	uint64_t d1Base;
