@@ -37,6 +37,9 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <map>
+#include <memory>
+#include <mutex>
 #include <string>
 
 #include <nemo_b200.h>
@@ -173,6 +176,14 @@ k_gather_out(Net n, int nnzRec, const float* w, float* wOut)
 	}
 }
 
+/* gu[t] of a neuron and trial from its u[t], gs[t] and gv[t] */
+__device__ __forceinline__ float guOf(const Net& n, float u, float gs, float gv)
+{
+	const float a = __fadd_rn(1.0f, __fmul_rn(n.kappa, fabsf(__fsub_rn(u, n.theta))));
+	const float sp = __fdiv_rn(1.0f, __fmul_rn(a, a));
+	return __fadd_rn(__fmul_rn(sp, __fsub_rn(gs, __fmul_rn(n.theta, gv))), gv);
+}
+
 /* One backward step: gu[t] of every neuron j from gu[t+1] (guNext, [N][32])
  * and u[t] (uSeg). Warp per neuron (source view), lane per trial; wOut: the
  * recurrent weights in out-synapse order. A chunk's 32 rows of guNext are
@@ -211,10 +222,7 @@ k_back(Net n, int t, const float* wOut, const float* uSeg, int segStart, const f
 			}
 			gv = __fmul_rn(n.beta, guNext[cell]);
 		}
-		const float u = uSeg[(size_t(t - segStart) * n.N) * 32 + cell];
-		const float a = __fadd_rn(1.0f, __fmul_rn(n.kappa, fabsf(__fsub_rn(u, n.theta))));
-		const float sp = __fdiv_rn(1.0f, __fmul_rn(a, a));
-		const float gu = __fadd_rn(__fmul_rn(sp, __fsub_rn(gs, __fmul_rn(n.theta, gv))), gv);
+		const float gu = guOf(n, uSeg[(size_t(t - segStart) * n.N) * 32 + cell], gs, gv);
 		guOut[(size_t(t - segStart) * n.N) * 32 + cell] = active ? gu : 0.0f;
 	}
 }
@@ -251,9 +259,7 @@ k_dw_relaxed(Net n, int segStart, int segEnd, const float* guSeg, const float* s
  * spikes are known, so each unit's (step, trial) pairs of the segment are
  * listed once (k_events) and every synapse walks its unit's list: the work is
  * the number of spikes times the fan-out, where walking words tests every
- * (step, synapse) word and shuffles every one that is not 0 (a gradient step
- * of 10,000 neurons, 2.5e6 synapses, 500 steps and 32 trials on a B200: 62.4 ms
- * with a launch per recomputed step, 48.5 with the lists). A segment is
+ * (step, synapse) word and shuffles every one that is not 0. A segment is
  * taken in parts of at most PART_STEPS steps, the most for which a neuron's
  * currents of all steps and trials stay in shared memory (8 KB a warp) and a
  * code step * 32 + trial fits 16 bits. */
@@ -319,65 +325,84 @@ k_events(Net n, int c0, int c1, int L, const uint32_t* sBits, const uint32_t* in
 }
 
 /* The steps [t0, t1) (one part) from v before them (vIn): u of every step
- * into uOut (segment buffer [K][N][32]), v after them into vOut. Warp per
+ * into uOut (segment buffer [K][N][tw]), v after them into vOut. Warp per
  * neuron: its currents of all steps and trials are accumulated in shared
- * memory, synapse after synapse in order, a synapse's events over the lanes
- * (distinct cells); a cell so gets its weights in synapse order, as in the
+ * memory, synapse after synapse in order, a synapse's events over the lanes,
+ * two a lane (distinct cells); a cell so gets its weights in synapse order, as in the
  * forward, and u is bit-identical. The codes of the next synapses are loaded
  * while the last ones are added. */
 __global__ void __launch_bounds__(PART_WARPS * 32)
-k_recompute(Net n, int t0, int t1, int segStart, int L, const float* w, const uint16_t* codes, const uint32_t* cnt,
-		const float* vIn, float* vOut, float* uOut)
+k_recompute(Net n, int tw, int t0, int t1, int segStart, int L, const float* w, const uint16_t* codes,
+		const uint32_t* cnt, const float* vIn, float* vOut, float* uOut)
 {
 	extern __shared__ float sCur[];
 	const int U = 4;
 	const uint32_t lane = threadIdx.x & 31u;
 	const bool active = lane < uint32_t(n.B);
-	float* cur = sCur + size_t(threadIdx.x >> 5) * (size_t(L) * 32);
 	const size_t cap = size_t(L) * 32;
+	float* cur = sCur + size_t(threadIdx.x >> 5) * (cap + 32);
 	const int len = t1 - t0;
 	const int warps = int((gridDim.x * blockDim.x) >> 5);
 	for(int i = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n.N; i += warps) {
 		for(int r = 0; r < len; ++r) cur[r * 32 + int(lane)] = 0.0f;
 		__syncwarp();
 		const int k0 = n.rowptr[i], k1 = n.rowptr[i + 1];
+		/* the synapses of a group of 32, and those of the next one on their way:
+		 * unit and weight during the first half, the unit's count during the
+		 * second (past the end: a count of 0) */
+		int p = k0 + int(lane) < k1 ? n.pre[k0 + int(lane)] : 0;
+		float wk = k0 + int(lane) < k1 ? w[k0 + int(lane)] : 0.0f;
+		uint32_t ck = k0 + int(lane) < k1 ? cnt[p] : 0u;
 		for(int base = k0; base < k1; base += 32) {
-			const int k = base + int(lane);
-			const int p = k < k1 ? n.pre[k] : 0;
-			const float wk = k < k1 ? w[k] : 0.0f;
-			const uint32_t ck = k < k1 ? cnt[p] : 0u;
-			const int nk = min(32, k1 - base);
+			const int k = base + 32 + int(lane);
+			int pNext = 0;
+			float wNext = 0.0f;
+			uint32_t cNext = 0;
+			if(k < k1) {
+				pNext = n.pre[k];
+				wNext = w[k];
+			}
 			uint32_t next[U];
 #pragma unroll
 			for(int x = 0; x < U; ++x) {
 				const uint32_t c = __shfl_sync(FULL, ck, x);
 				const int pq = __shfl_sync(FULL, p, x);
-				next[x] = lane < c ? codes[size_t(pq) * cap + lane] : 0u;
+				next[x] = 2u * lane < c ? *reinterpret_cast<const uint32_t*>(codes + size_t(pq) * cap + 2u * lane) : 0u;
 			}
-			for(int q0 = 0; q0 < nk; q0 += U) {
+#pragma unroll 1
+			for(int q0 = 0; q0 < 32; q0 += U) {
+				if(q0 == 16 && k < k1) cNext = cnt[pNext];
 				uint32_t code[U];
 #pragma unroll
 				for(int x = 0; x < U; ++x) {
 					code[x] = next[x];
 					const int q = (q0 + U + x) & 31;
-					const uint32_t c = q0 + U + x < nk ? __shfl_sync(FULL, ck, q) : 0u;
+					const uint32_t c = q0 + U < 32 ? __shfl_sync(FULL, ck, q) : 0u;
 					const int pq = __shfl_sync(FULL, p, q);
-					next[x] = lane < c ? codes[size_t(pq) * cap + lane] : 0u;
+					next[x] = 2u * lane < c ? *reinterpret_cast<const uint32_t*>(codes + size_t(pq) * cap + 2u * lane) : 0u;
 				}
 #pragma unroll
 				for(int x = 0; x < U; ++x) {
-					/* past the last synapse: a count of 0 */
 					const int q = q0 + x;
 					const uint32_t c = __shfl_sync(FULL, ck, q);
 					const float wq = __shfl_sync(FULL, wk, q);
-					if(lane < c) cur[code[x]] = __fadd_rn(cur[code[x]], wq);
-					if(c > 32u) {
+					/* distinct cells: both loads, then both stores; past the end
+					 * of the list the cell that is never read */
+					float* a = cur + (2u * lane < c ? code[x] & 0xffffu : uint32_t(cap));
+					float* b = cur + (2u * lane + 1u < c ? code[x] >> 16 : uint32_t(cap));
+					const float va = *a, vb = *b;
+					*a = __fadd_rn(va, wq);
+					*b = __fadd_rn(vb, wq);
+					if(c > 64u) {
 						const uint16_t* more = codes + size_t(__shfl_sync(FULL, p, q)) * cap;
-						for(uint32_t e = 32u + lane; e < c; e += 32u) cur[more[e]] = __fadd_rn(cur[more[e]], wq);
+						for(uint32_t e = 64u + lane; e < c; e += 32u) cur[more[e]] = __fadd_rn(cur[more[e]], wq);
 					}
 					__syncwarp();
 				}
 			}
+			p = pNext;
+			wk = wNext;
+			ck = cNext;
 		}
 		const size_t cell = size_t(i) * 32 + lane;
 		float v = vIn[cell];
@@ -385,7 +410,7 @@ k_recompute(Net n, int t0, int t1, int segStart, int L, const float* w, const ui
 			const float u = __fadd_rn(__fmul_rn(n.beta, v), cur[r * 32 + int(lane)]);
 			const float s = (active && u >= n.theta) ? 1.0f : 0.0f;
 			v = __fsub_rn(u, __fmul_rn(n.theta, s));
-			uOut[(size_t(t0 - segStart + r) * n.N) * 32 + cell] = u;
+			if(int(lane) < tw) uOut[(size_t(t0 - segStart + r) * n.N + i) * tw + lane] = u;
 		}
 		vOut[cell] = v;
 		__syncwarp();
@@ -397,8 +422,8 @@ k_recompute(Net n, int t0, int t1, int segStart, int L, const float* w, const ui
  * gu over its presynaptic unit's events, by step, then by trial, eight codes
  * a load. */
 __global__ void __launch_bounds__(PART_WARPS * 32)
-k_dw_events(Net n, int t0, int t1, int segStart, int L, const float* guSeg, const uint16_t* codes, const uint32_t* cnt,
-		float* dw)
+k_dw_events(Net n, int tw, int t0, int t1, int segStart, int L, const float* guSeg, const uint16_t* codes,
+		const uint32_t* cnt, const unsigned* error, float* dw)
 {
 	extern __shared__ float sGu[];
 	const uint32_t lane = threadIdx.x & 31u;
@@ -406,22 +431,32 @@ k_dw_events(Net n, int t0, int t1, int segStart, int L, const float* guSeg, cons
 	float* g = sGu + size_t(threadIdx.x >> 5) * (cap + 32);
 	const int len = t1 - t0;
 	const int warps = int((gridDim.x * blockDim.x) >> 5);
+	/* a barrier of the adjoint gave up: the result is NaN */
+	const float zero = *error ? __int_as_float(0x7fffffff) : 0.0f;
 	g[cap + lane] = 0.0f;
 	for(int i = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n.N; i += warps) {
 		for(int r = 0; r < len; ++r) {
-			g[r * 32 + int(lane)] = guSeg[(size_t(t0 - segStart + r) * n.N + i) * 32 + lane];
+			g[r * 32 + int(lane)] = int(lane) < tw ? guSeg[(size_t(t0 - segStart + r) * n.N + i) * tw + lane] : 0.0f;
 		}
 		__syncwarp();
 		const int k0 = n.rowptr[i], k1 = n.rowptr[i + 1];
-		for(int k = k0 + int(lane); k < k1; k += 32) {
-			const int p = n.pre[k];
-			const uint32_t c = cnt[p];
+		/* the next synapse's unit, count and first codes are on their way while
+		 * one is summed */
+		int k = k0 + int(lane);
+		int p = k < k1 ? n.pre[k] : 0;
+		uint32_t c = k < k1 ? cnt[p] : 0u;
+		int pNext = k + 32 < k1 ? n.pre[k + 32] : 0;
+		for(; k < k1; k += 32) {
 			const uint4* list = reinterpret_cast<const uint4*>(codes + size_t(p) * cap);
-			float acc = 0.0f;
-			uint4 next = c ? list[0] : make_uint4(0u, 0u, 0u, 0u);
+			float acc = zero;
+			uint4 n0 = list[0], n1 = list[1];
+			const uint32_t cNext = k + 32 < k1 ? cnt[pNext] : 0u;
+			const int pAfter = k + 64 < k1 ? n.pre[k + 64] : 0;
+			const float old = dw[k];
 			for(uint32_t e = 0; e < c; e += 8u) {
-				const uint4 x = next;
-				if(e + 8u < c) next = list[(e >> 3) + 1u];
+				const uint4 x = n0;
+				n0 = n1;
+				if(e + 16u < c) n1 = list[(e >> 3) + 2u];
 				acc = __fadd_rn(acc, g[x.x & 0xffffu]);
 				acc = __fadd_rn(acc, g[x.x >> 16]);
 				acc = __fadd_rn(acc, g[x.y & 0xffffu]);
@@ -431,9 +466,474 @@ k_dw_events(Net n, int t0, int t1, int segStart, int L, const float* guSeg, cons
 				acc = __fadd_rn(acc, g[x.w & 0xffffu]);
 				acc = __fadd_rn(acc, g[x.w >> 16]);
 			}
-			dw[k] = __fadd_rn(dw[k], acc);
+			dw[k] = __fadd_rn(old, acc);
+			p = pNext;
+			c = cNext;
+			pNext = pAfter;
 		}
 		__syncwarp();
+	}
+}
+
+/* floats of a row of trials: 8, 16 or 32 */
+static int rowWidth(int B) { return B <= 8 ? 8 : (B <= 16 ? 16 : 32); }
+
+/* ---- the adjoint of a segment in one launch (spikes as bits) ----
+ *
+ * A step is gs_j = sum over out-synapses (j -> i) of w * gu[t+1]_i: every
+ * synapse reads one row of gu (4 bytes a trial). From L2 that is 256 MB a
+ * step for 2e6 synapses and 32 trials, a chain of dependent row gathers a
+ * warp (71 us a step). Here the rows are in shared memory, read at 128 bytes
+ * a clock and SM:
+ *   - the blocks form groups of `parts` blocks (8, or as many as the rows
+ *     need); block p of each holds the rows of the p-th part of the neurons,
+ *     and every group owns an equal share of the sources, so that each
+ *     (source, part) pair has one block;
+ *   - a source is worked off by a few lanes (of 32 trials: four lanes, two
+ *     float4 each, so that a warp has 8 sources and reads their rows without
+ *     bank conflicts), which walk the pair's synapses in order, four a turn. The
+ *     synapses are laid out part by part, in a part source by source, as
+ *     {row offset, weight} (k_out_fill), every pair filled up to whole turns,
+ *     and a lane group has a run of whole sources of about the same length as
+ *     every other: the groups of a warp go in step and nothing in a turn is a
+ *     branch (a divergent one costs about 75 clocks). A block keeps its
+ *     synapses in shared memory when they fit, else they come through a ring
+ *     of asynchronous copies a lane group;
+ *   - a source's sum over one part goes to global memory (L2) at its last
+ *     entry; after a grid barrier the parts are added, in part order, so that
+ *     the result does not depend on timing, by the block that finishes the
+ *     source and writes its gu[t] row; a second grid barrier ends the step.
+ *     (Thread-block clusters of 8 with the sums in distributed shared memory
+ *     measured slower: 15 of them run at once, 120 of 148 SMs, their barrier
+ *     is no cheaper, and reading the sums took twice as long as from L2.) */
+
+const int ADJ_THREADS = 1024;
+const int ADJ_WARPS = ADJ_THREADS / 32;
+const int ADJ_MIN_PARTS = 8, ADJ_MAX_PARTS = 32;
+/* sources of a group (their places in a block's shared memory) */
+const size_t ADJ_SOURCES = 8192;
+/* rows of gu, the group's sources and the rings (the largest block has 227
+ * KB) */
+const size_t ADJ_SMEM = 224 * 1024;
+/* entries a block may load past its last bucket's end (its rings) */
+const size_t ADJ_SLACK = 64;
+/* in a bucket's last entry's row offset (a multiple of 32) */
+const uint32_t ADJ_LAST = 1u;
+
+struct Adjoint {
+	int c0, c1;              /* the segment's steps */
+	int parts;               /* blocks per group */
+	int partRows;            /* neurons per part */
+	int perGroup;            /* sources per group */
+	const uint2* bucket;     /* [parts][N] {first entry in the part, count} */
+	const uint32_t* total;   /* [parts] entries of each part */
+	const uint2* entries;    /* {byte offset of the target's row in its part (| ADJ_LAST), weight}, part after part */
+	float* sums;             /* [parts][N][TW] */
+	const float* uSeg;       /* [K][N][TW] */
+	const float* guNext;     /* [N][TW] gu of step c1 */
+	float* guSeg;            /* [K][N][TW] */
+	const float* dcounts;
+	unsigned* barrier;       /* [0] arrivals, [1] error */
+	unsigned barrierBase;    /* arrivals before this launch */
+};
+
+/* Synapses of every (source, part) pair, warp per source: cnt[p * N + j] */
+__global__ void __launch_bounds__(THREADS)
+k_out_count(Net n, int parts, int partRows, uint2* bucket)
+{
+	const uint32_t lane = threadIdx.x & 31u;
+	const int warps = int((gridDim.x * blockDim.x) >> 5);
+	for(int j = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5); j < n.N; j += warps) {
+		uint32_t mine = 0;   /* lane p: the count of part p */
+		const int e0 = n.colptr[j], e1 = n.colptr[j + 1];
+		for(int base = e0; base < e1; base += 32) {
+			const int e = base + int(lane);
+			const int part = e < e1 ? n.post[e] / partRows : -1;
+			for(int p = 0; p < parts; ++p) {
+				const uint32_t c = uint32_t(__popc(__ballot_sync(FULL, part == p)));
+				if(int(lane) == p) mine += c;
+			}
+		}
+		if(int(lane) < parts) bucket[size_t(lane) * n.N + j].y = mine;
+	}
+}
+
+/* The first entry of every pair in its part (block per part): an exclusive
+ * sum of the counts rounded up to a multiple of 4 (at least 4), which
+ * k_out_fill fills up with entries that add 0 (the row past the part's last
+ * one, weight 0) */
+__global__ void __launch_bounds__(1024)
+k_out_scan(int N, uint2* bucket, uint32_t* total)
+{
+	__shared__ uint32_t warpSum[32];
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	uint2* b = bucket + size_t(blockIdx.x) * N;
+	const int per = (N + 1023) / 1024;
+	const int lo = min(N, int(threadIdx.x) * per), hi = min(N, lo + per);
+	uint32_t sum = 0;
+	for(int j = lo; j < hi; ++j) sum += max(4u, (b[j].y + 3u) & ~3u);
+	uint32_t incl = sum;
+#pragma unroll
+	for(int d = 1; d < 32; d <<= 1) {
+		const uint32_t x = __shfl_up_sync(FULL, incl, d);
+		if(lane >= uint32_t(d)) incl += x;
+	}
+	if(lane == 31) warpSum[warp] = incl;
+	__syncthreads();
+	if(warp == 0) {
+		const uint32_t v = warpSum[lane];
+		uint32_t w = v;
+#pragma unroll
+		for(int d = 1; d < 32; d <<= 1) {
+			const uint32_t x = __shfl_up_sync(FULL, w, d);
+			if(lane >= uint32_t(d)) w += x;
+		}
+		warpSum[lane] = w - v;
+		if(lane == 31) total[blockIdx.x] = w;
+	}
+	__syncthreads();
+	uint32_t run = warpSum[warp] + incl - sum;
+	for(int j = lo; j < hi; ++j) {
+		b[j].x = run;
+		run += max(4u, (b[j].y + 3u) & ~3u);
+	}
+}
+
+/* The entries of every source (warp per source), in out-synapse order within
+ * a pair */
+__global__ void __launch_bounds__(THREADS)
+k_out_fill(Net n, int parts, int partRows, int rowBytes, const uint2* bucket, const uint32_t* total, const float* w,
+		uint2* entries)
+{
+	const uint32_t lane = threadIdx.x & 31u;
+	const uint32_t lt = (1u << lane) - 1u;
+	const int warps = int((gridDim.x * blockDim.x) >> 5);
+	uint32_t partBase = 0;   /* lane p: the first entry of part p */
+	for(int p = 0; p < int(lane) && p < parts; ++p) partBase += total[p];
+	for(int j = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5); j < n.N; j += warps) {
+		uint32_t next = int(lane) < parts ? partBase + bucket[size_t(lane) * n.N + j].x : 0u;
+		const int e0 = n.colptr[j], e1 = n.colptr[j + 1];
+		for(int base = e0; base < e1; base += 32) {
+			const int e = base + int(lane);
+			const int i = e < e1 ? n.post[e] : 0;
+			const int part = e < e1 ? i / partRows : -1;
+			for(int p = 0; p < parts; ++p) {
+				const uint32_t m = __ballot_sync(FULL, part == p);
+				const uint32_t first = __shfl_sync(FULL, next, p);
+				if(part == p) {
+					entries[first + uint32_t(__popc(m & lt))] = make_uint2(uint32_t(i - p * partRows) * uint32_t(rowBytes),
+							__float_as_uint(w[n.wpos[e]]));
+				}
+				if(int(lane) == p) next += uint32_t(__popc(m));
+			}
+		}
+		__syncwarp();
+		if(int(lane) < parts) {
+			const uint32_t first = partBase + bucket[size_t(lane) * n.N + j].x;
+			while(next == first || (next & 3u)) entries[next++] = make_uint2(uint32_t(partRows) * uint32_t(rowBytes), 0u);
+			entries[next - 1u].x |= ADJ_LAST;
+		}
+	}
+}
+
+/* The grid barrier: every block arrives (its writes before are visible to
+ * what waits), then waits for `target` arrivals in all. The wait is bounded:
+ * after 10 s it sets the error word (the call's results become NaN), and no
+ * block waits any more. */
+__device__ __forceinline__ void gridArrive(unsigned* bar)
+{
+	__syncthreads();
+	if(threadIdx.x == 0) {
+		asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(__cvta_generic_to_global(bar)) : "memory");
+	}
+}
+
+__device__ __forceinline__ void gridWait(unsigned* bar, unsigned target)
+{
+	if(threadIdx.x == 0) {
+		const size_t g = __cvta_generic_to_global(bar);
+		unsigned long long start = 0;
+		for(unsigned spins = 1;; ++spins) {
+			unsigned v;
+			asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(g) : "memory");
+			if(int(v - target) >= 0) break;
+			if((spins & 255u) == 0) {
+				unsigned long long now;
+				asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+				if(start == 0) start = now;
+				if(*(volatile unsigned*) &bar[1]) break;
+				if(now - start > 10ull * 1000 * 1000 * 1000) {
+					*(volatile unsigned*) &bar[1] = 1u;
+					break;
+				}
+			}
+		}
+	}
+	__syncthreads();
+}
+
+/* Row-width constants of k_adjoint */
+template<int TW>
+struct AdjointShape {
+	static const int FLOATS = TW == 32 ? 8 : 4;     /* trials of a lane */
+	static const int LANES = TW / FLOATS;           /* lanes of a source */
+	static const int GROUPS = 32 / LANES;           /* sources of a warp at once */
+	static const int SLOTS = ADJ_WARPS * GROUPS;    /* sources of a block at once */
+	static const int RING = 8;                      /* entry pairs on their way to a lane group */
+};
+
+/* bytes of the rings of a block */
+static size_t
+adjointRings(int tw)
+{
+	const int slots = tw == 32 ? AdjointShape<32>::SLOTS : (tw == 16 ? AdjointShape<16>::SLOTS : AdjointShape<8>::SLOTS);
+	return size_t(slots) * AdjointShape<32>::RING * 16;
+}
+
+/* Parts of the neurons: 8, or as many as it takes for a part's rows (and the
+ * row of zeros) to fit a block beside its sources and rings; 0 past 32 parts
+ * (40,000 neurons of 32 trials) */
+static int
+adjointParts(int N, int tw)
+{
+	for(int parts = ADJ_MIN_PARTS; parts <= ADJ_MAX_PARTS; ++parts) {
+		const size_t rows = size_t((N + parts - 1) / parts) + 1;
+		if(rows * tw * 4 + ADJ_SOURCES * 4 + adjointRings(tw) <= ADJ_SMEM) return parts;
+	}
+	return 0;
+}
+
+template<int TW>
+__global__ void __launch_bounds__(ADJ_THREADS, 1)
+k_adjoint(const __grid_constant__ Net n, const __grid_constant__ Adjoint a)
+{
+	extern __shared__ __align__(128) char smem[];
+	typedef AdjointShape<TW> S;
+	const int LANES = S::LANES, RING = S::RING, FLOATS = S::FLOATS;
+	const int Q = TW / 4;                     /* float4s of a row */
+	const uint32_t lane = threadIdx.x & 31u;
+	const int warp = int(threadIdx.x >> 5);
+	const int part = int(blockIdx.x) % a.parts;
+	/* the part's rows of gu and a row of zeros */
+	float* sG = reinterpret_cast<float*>(smem);
+	uint32_t* sFirst = reinterpret_cast<uint32_t*>(sG + size_t(a.partRows + 1) * TW);   /* first pair of each source */
+	uint4* sEntry = reinterpret_cast<uint4*>(sFirst + (a.perGroup + 1 + 3) / 4 * 4);
+	const uint32_t room = uint32_t(ADJ_SMEM - size_t(reinterpret_cast<char*>(sEntry) - smem)) / 16u;
+
+	const int src0 = int(blockIdx.x) / a.parts * a.perGroup;
+	const int ns = max(0, min(a.perGroup, n.N - src0));         /* the group's sources */
+	const int row0 = part * a.partRows;
+	const int rows = max(0, min(a.partRows, n.N - row0));       /* the block's rows */
+	const int own = (a.perGroup + a.parts - 1) / a.parts;       /* sources a block finishes */
+	const int fin0 = min(ns, part * own), fin1 = min(ns, fin0 + own);
+	const int items = (fin1 - fin0) * Q;
+	uint32_t partBase = 0;
+	for(int p = 0; p < part; ++p) partBase += a.total[p];
+	const uint2* bucket = a.bucket + size_t(part) * n.N + src0;
+	const uint32_t firstPair = ns ? bucket[0].x / 2u : 0u;
+	for(int s = int(threadIdx.x); s < ns; s += ADJ_THREADS) {
+		const uint2 b = bucket[s];
+		sFirst[s] = b.x / 2u - firstPair;
+		if(s == ns - 1) sFirst[ns] = b.x / 2u - firstPair + max(4u, (b.y + 3u) & ~3u) / 2u;
+	}
+	if(threadIdx.x < uint32_t(TW)) sG[size_t(a.partRows) * TW + threadIdx.x] = 0.0f;
+	__syncthreads();
+	/* the block's entries in pairs, one run for its sources in order */
+	const uint32_t pairs = ns ? sFirst[ns] : 0u;
+	const uint4* entries = reinterpret_cast<const uint4*>(a.entries + partBase) + firstPair;
+	const bool kept = pairs + 2u <= room;   /* and two pairs of slack */
+	if(kept) {
+		for(uint32_t q = threadIdx.x; q < pairs; q += ADJ_THREADS) sEntry[q] = __ldg(entries + q);
+	}
+
+	/* the lane group's run: the sources that start in its share of the pairs.
+	 * A 16-byte load costs a warp the same with one group as with all, so the
+	 * groups used fill whole warps: one for a source, from 128 sources on one
+	 * for at least five (runs of five sources differ little in length) */
+	const int group = int(lane) / LANES;
+	const int slot = warp * S::GROUPS + group;
+	const int used = min(S::SLOTS, ns <= 128 ? max(ns, 1) : max(128, ns / 5));
+	auto sourceAt = [&](uint64_t pair) {
+		int lo = 0, hi = ns;   /* the first source that starts at or after it */
+		while(lo < hi) {
+			const int mid = (lo + hi) / 2;
+			if(uint64_t(sFirst[mid]) >= pair) hi = mid;
+			else lo = mid + 1;
+		}
+		return lo;
+	};
+	int s0 = ns, s1 = ns;
+	if(ns <= 128) {
+		s0 = min(slot, ns);
+		s1 = min(slot + 1, ns);
+	} else if(slot < used) {
+		s0 = sourceAt((uint64_t(pairs) * slot + used - 1) / used);
+		s1 = sourceAt((uint64_t(pairs) * (slot + 1) + used - 1) / used);
+	}
+	const uint32_t run0 = s0 < s1 ? sFirst[s0] : 0u;
+	const uint32_t turns = s0 < s1 ? (sFirst[s1] - run0) / 2u : 0u;
+	const uint32_t live = __ballot_sync(FULL, turns != 0u);   /* the lanes with a run */
+	const int own0 = int(lane) % LANES;
+	/* the lane's float4s of a row: odd groups start with the second one, so
+	 * that the two groups of a quarter-warp meet on no bank */
+	const int H = FLOATS / 4;
+	int at[H];
+#pragma unroll
+	for(int h = 0; h < H; ++h) at[h] = H == 1 ? own0 * 16 : ((h + group) % H) * 64 + own0 * 16;
+	const char* const rowsAt = reinterpret_cast<const char*>(sG);
+	const uint32_t zeroAt = uint32_t(a.partRows) * TW * 4u;
+	uint4* ring = sEntry + (warp * S::GROUPS + group) * RING;
+	const uint32_t ringAt = uint32_t(__cvta_generic_to_shared(ring));
+	float* const sums0 = a.sums + (size_t(part) * n.N + size_t(src0 + s0)) * TW;
+	const int bins = n.T / n.binSteps;
+	unsigned target = a.barrierBase;
+
+	auto fetch = [&](uint32_t pair) {
+		asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(ringAt + (pair & uint32_t(RING - 1)) * 16u),
+				"l"(__cvta_generic_to_global(entries + pair)) : "memory");
+	};
+	__syncthreads();
+
+	for(int t = a.c1 - 1; t >= a.c0; --t) {
+		const bool last = t == n.T - 1;
+		const float* next = t == a.c1 - 1 ? a.guNext : a.guSeg + size_t(t + 1 - a.c0) * n.N * TW;
+		const float* uT = a.uSeg + size_t(t - a.c0) * n.N * TW;
+		float* out = a.guSeg + size_t(t - a.c0) * n.N * TW;
+
+		if(!last) {
+			if(!kept && turns) {
+				for(int q = own0; q < RING; q += LANES) fetch(run0 + uint32_t(q));
+			}
+			/* the rows of gu[t+1], past the L1 cache: other blocks have written
+			 * them */
+			const uint32_t dst = uint32_t(__cvta_generic_to_shared(sG));
+			const char* src = reinterpret_cast<const char*>(next + size_t(row0) * TW);
+			for(int q = int(threadIdx.x); q < rows * Q; q += ADJ_THREADS) {
+				asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + uint32_t(q) * 16u),
+						"l"(__cvta_generic_to_global(src + size_t(q) * 16)) : "memory");
+			}
+			asm volatile("cp.async.wait_all;" ::: "memory");
+			__syncthreads();
+			if(turns) {
+				const uint32_t most = __reduce_max_sync(live, turns);
+				uint32_t pos = run0, filled = run0 + uint32_t(RING);
+				float acc[FLOATS];
+#pragma unroll
+				for(int q = 0; q < FLOATS; ++q) acc[q] = 0.0f;
+				/* one entry into the lane's sums; `on` (all bits or none) sends
+				 * those of a group that is through to the row of zeros */
+				auto add = [&](uint32_t off, uint32_t w, uint32_t on) {
+					const char* row = rowsAt + ((off & on & ~31u) | (zeroAt & ~on));
+					const float ww = __uint_as_float(w & on);
+#pragma unroll
+					for(int h = 0; h < H; ++h) {
+						const float4 g = *reinterpret_cast<const float4*>(row + at[h]);
+						acc[4 * h + 0] = __fmaf_rn(ww, g.x, acc[4 * h + 0]);
+						acc[4 * h + 1] = __fmaf_rn(ww, g.y, acc[4 * h + 1]);
+						acc[4 * h + 2] = __fmaf_rn(ww, g.z, acc[4 * h + 2]);
+						acc[4 * h + 3] = __fmaf_rn(ww, g.w, acc[4 * h + 3]);
+					}
+				};
+				size_t sumAt = __cvta_generic_to_global(sums0);
+				auto turn = [&](uint32_t e, const uint4& x, const uint4& y) {
+					const uint32_t on = e < turns ? FULL : 0u;
+					add(x.x, x.y, on);
+					add(x.z, x.w, on);
+					add(y.x, y.y, on);
+					add(y.z, y.w, on);
+					pos += on & 2u;
+					/* the source's last entry: its sum, then the next one's */
+					const uint32_t done = y.z & on & ADJ_LAST;
+#pragma unroll
+					for(int h = 0; h < H; ++h) {
+						asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t"
+								"@p st.global.v4.f32 [%0], {%1, %2, %3, %4};\n\t}" :: "l"(sumAt + size_t(at[h])),
+								"f"(acc[4 * h]), "f"(acc[4 * h + 1]), "f"(acc[4 * h + 2]), "f"(acc[4 * h + 3]), "r"(done) : "memory");
+					}
+					const uint32_t keep = done - 1u;   /* all bits, or none after the last */
+#pragma unroll
+					for(int q = 0; q < FLOATS; ++q) acc[q] = __uint_as_float(__float_as_uint(acc[q]) & keep);
+					sumAt += done * uint32_t(TW * 4);
+				};
+				if(kept) {
+					/* a group that is through may read past its run: inside the
+					 * block's entries and the slack behind them */
+					for(uint32_t e = 0; e < most; ++e) turn(e, sEntry[pos], sEntry[pos + 1u]);
+				} else {
+					/* two pairs are used and replaced a turn; this turn's were
+					 * asked for RING / 2 - 1 turns ago at the latest */
+					for(uint32_t e = 0; e < most; ++e) {
+						const uint32_t upTo = pos + uint32_t(RING);
+						if(filled + uint32_t(own0) < upTo) fetch(filled + uint32_t(own0));
+						filled = upTo;
+						asm volatile("cp.async.commit_group;\n\tcp.async.wait_group %0;" :: "n"(RING / 2 - 1) : "memory");
+						__syncwarp(live);
+						turn(e, ring[pos & uint32_t(RING - 1)], ring[(pos + 1u) & uint32_t(RING - 1)]);
+						__syncwarp(live);
+					}
+				}
+			}
+		}
+		gridArrive(a.barrier);
+		/* what finishing the thread's first item needs, on its way during the
+		 * barrier (a thread without an item loads some row: a load under a
+		 * condition would be waited for at the condition's end) */
+		float4 u0, g0;
+		float dc[4];
+		auto operands = [&](int x, float4& u, float4& g) {
+			const size_t cell = size_t(min(src0 + fin0 + x / Q, n.N - 1)) * TW + size_t(x % Q) * 4;
+			u = *reinterpret_cast<const float4*>(uT + cell);
+			g = __ldcg(reinterpret_cast<const float4*>(next + cell));
+		};
+		operands(min(int(threadIdx.x), max(items - 1, 0)), u0, g0);
+#pragma unroll
+		for(int q = 0; q < 4; ++q) {
+			const int b = min(int(threadIdx.x) % Q * 4 + q, n.B - 1);
+			dc[q] = __ldg(&a.dcounts[size_t(b) * bins + t / n.binSteps]);
+		}
+		target += gridDim.x;
+		gridWait(a.barrier, target);
+#pragma unroll 1
+		for(int x = int(threadIdx.x); x < items; x += ADJ_THREADS) {
+			if(x >= ADJ_THREADS) operands(x, u0, g0);
+			const int c = (x % Q) * 4;
+			const size_t cell = size_t(src0 + fin0 + x / Q) * TW + c;
+			float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+			if(last) {
+				g0 = sum;
+			} else {
+				for(int q0 = 0; q0 < a.parts; q0 += 8) {
+					float4 y[8];
+#pragma unroll
+					for(int q = 0; q < 8; ++q) {
+						y[q] = __ldcg(reinterpret_cast<const float4*>(a.sums + size_t(min(q0 + q, a.parts - 1)) * n.N * TW + cell));
+					}
+#pragma unroll
+					for(int q = 0; q < 8; ++q) {
+						if(q0 + q < a.parts) {
+							sum.x = __fadd_rn(sum.x, y[q].x);
+							sum.y = __fadd_rn(sum.y, y[q].y);
+							sum.z = __fadd_rn(sum.z, y[q].z);
+							sum.w = __fadd_rn(sum.w, y[q].w);
+						}
+					}
+				}
+			}
+			const float us[4] = {u0.x, u0.y, u0.z, u0.w}, gn[4] = {g0.x, g0.y, g0.z, g0.w}, ss[4] = {sum.x, sum.y, sum.z, sum.w};
+			float r[4];
+#pragma unroll
+			for(int q = 0; q < 4; ++q) {
+				r[q] = guOf(n, us[q], __fadd_rn(dc[q], ss[q]), __fmul_rn(n.beta, gn[q]));
+				if(c + q >= n.B) r[q] = 0.0f;
+			}
+			const float4 v = make_float4(r[0], r[1], r[2], r[3]);
+			*reinterpret_cast<float4*>(out + cell) = v;
+		}
+		if(t > a.c0) {
+			target += gridDim.x;
+			gridArrive(a.barrier);
+			gridWait(a.barrier, target);
+		}
 	}
 }
 
@@ -448,6 +948,109 @@ grid(int N)
 	const long cap = long(sms) * 8;
 	return int(blocks < cap ? blocks : cap);
 }
+
+static const void*
+adjointKernel(int tw)
+{
+	return tw == 8 ? (const void*) k_adjoint<8> : (tw == 16 ? (const void*) k_adjoint<16> : (const void*) k_adjoint<32>);
+}
+
+/* blocks of a kernel with that much shared memory that can run at once (one
+ * an SM; 0: it does not fit), by device and kernel */
+static int
+residentBlocks(const void* kernel, int threads, size_t smem)
+{
+	static std::mutex lock;
+	static std::map<std::pair<int, const void*>, int> known;
+	int dev = 0;
+	NEMO_CUDA(cudaGetDevice(&dev));
+	std::lock_guard<std::mutex> guard(lock);
+	const std::pair<int, const void*> key(dev, kernel);
+	auto it = known.find(key);
+	if(it != known.end()) return it->second;
+	int perSm = 0, sms = 0, coop = 0;
+	NEMO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+	NEMO_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+	if(coop && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
+		(void) cudaGetLastError();   /* a device with less shared memory */
+		coop = 0;
+	}
+	if(coop) NEMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, threads, smem));
+	known[key] = perSm > 0 ? sms : 0;
+	return known[key];
+}
+
+struct AdjointPlan {
+	int tw = 32;
+	int parts = 0;   /* 0: step by step (k_back) */
+	int groups = 0, partRows = 0, perGroup = 0;
+};
+
+/* The adjoint in one launch a segment, unless its rows ask for more parts than
+ * there are (adjointParts): a group for every 64 sources, as many as run at
+ * once. */
+static AdjointPlan
+planAdjoint(const Net& n)
+{
+	AdjointPlan p;
+	const int tw = rowWidth(n.B);
+	const int parts = adjointParts(n.N, tw);
+	const int most = residentBlocks(adjointKernel(tw), ADJ_THREADS, ADJ_SMEM);
+	if(parts == 0 || most < parts) return p;
+	const int groups = std::max(1, std::min(most / parts, (n.N + 63) / 64));
+	const int per = (n.N + groups - 1) / groups;
+	if(size_t(per) + 4 > ADJ_SOURCES) return p;
+	p.tw = tw;
+	p.parts = parts;
+	p.groups = (n.N + per - 1) / per;
+	p.partRows = (n.N + parts - 1) / parts;
+	p.perGroup = per;
+	return p;
+}
+
+/* A stream that is being captured (or cannot tell) takes the launches whose
+ * blocks never wait for one another: two graphs may run at once, and nothing
+ * then orders their launches (Turn). */
+static bool
+capturing(cudaStream_t st)
+{
+	cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+	if(cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+		(void) cudaGetLastError();
+		return true;
+	}
+	return status != cudaStreamCaptureStatusNone;
+}
+
+/* The kernels whose blocks wait for one another run one after another on a
+ * device, whatever their streams: a call's launches wait for the last such
+ * call's (two grids that each hold some of the SMs could otherwise each wait
+ * for blocks of their own that cannot start). Held from before the first
+ * launch to after the last. */
+class Turn {
+public:
+	explicit Turn(cudaStream_t st) : m_stream(st), m_guard(s_lock)
+	{
+		int dev = 0;
+		NEMO_CUDA(cudaGetDevice(&dev));
+		cudaEvent_t& e = s_event[dev];
+		if(e == nullptr) NEMO_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+		m_event = e;
+		NEMO_CUDA(cudaStreamWaitEvent(st, e, 0));
+	}
+	~Turn() { cudaEventRecord(m_event, m_stream); }
+	Turn(const Turn&) = delete;
+	Turn& operator=(const Turn&) = delete;
+
+private:
+	static std::mutex s_lock;
+	static std::map<int, cudaEvent_t> s_event;
+	cudaStream_t m_stream;
+	std::lock_guard<std::mutex> m_guard;
+	cudaEvent_t m_event;
+};
+std::mutex Turn::s_lock;
+std::map<int, cudaEvent_t> Turn::s_event;
 
 static void
 validate(const Net& n)
@@ -474,13 +1077,18 @@ using namespace nemo_b200;
 
 /* The work buffer: v state [N][32], gu of the step after the segment [N][32],
  * the segment's u and gu [K][N][32], the event lists of its parts (codes, then
- * counts), then the recurrent weights in out-synapse order [nnzRec]. Made
+ * counts); the adjoint's synapses (buckets, part totals, entries) and sums or, step by
+ * step, the recurrent weights in out-synapse order; the grid barrier. Made
  * from the buffer's start rounded up to 128 bytes (the size has the slack). */
 struct LifWork {
 	float *v, *guNext, *uSeg, *guSeg;
 	uint16_t* codes;
 	uint32_t* cnt;
-	float* wOut;
+	float* wOut;        /* shares the entries' place */
+	uint2 *bucket, *entries;
+	uint32_t* total;
+	float* sums;
+	unsigned* barrier;
 	size_t bytes;
 
 	LifWork(const lif::Net& n, float* base)
@@ -498,7 +1106,13 @@ struct LifWork {
 		const size_t Y = size_t(lif::parts(K));
 		codes = reinterpret_cast<uint16_t*>(take(Y * units * size_t(lif::partSteps(K)) * 32 * 2));
 		cnt = reinterpret_cast<uint32_t*>(take(Y * units * 4));
-		wOut = reinterpret_cast<float*>(take(size_t(n.nnzRec) * 4));
+		const size_t P = size_t(lif::adjointParts(n.N, lif::rowWidth(n.B)));
+		bucket = reinterpret_cast<uint2*>(take(P * n.N * 8));
+		total = reinterpret_cast<uint32_t*>(take(P * 4));
+		entries = reinterpret_cast<uint2*>(take((size_t(n.nnzRec) + 4 * P * n.N + lif::ADJ_SLACK) * 8));
+		wOut = reinterpret_cast<float*>(entries);
+		sums = reinterpret_cast<float*>(take(P * n.N * lif::rowWidth(n.B) * 4));
+		barrier = reinterpret_cast<unsigned*>(take(8));
 		bytes = size_t(p - p0) + align;
 	}
 };
@@ -533,7 +1147,8 @@ nemo_b200_lif_forward(const nemo_b200_lif_net* net, const float* w, const uint32
 		memcpy(&n, net, sizeof(n));
 		lif::validate(n);
 		cudaStream_t st = static_cast<cudaStream_t>(stream);
-		float* v = LifWork(n, work).v;
+		const LifWork k(n, work);
+		float* v = k.v;
 		NEMO_CUDA(cudaMemsetAsync(v, 0, size_t(n.N) * 32 * 4, st));
 		NEMO_CUDA(cudaMemsetAsync(counts, 0, size_t(n.B) * (n.T / n.binSteps) * 4, st));
 		const int g = lif::grid(n.N);
@@ -563,16 +1178,39 @@ nemo_b200_lif_backward(const nemo_b200_lif_net* net, const float* w, const uint3
 		const size_t NS = size_t(n.N) * 32;
 		const LifWork k(n, work);
 		const int g = lif::grid(n.N);
-		/* the recurrent weights in out-synapse order, for k_back */
-		if(n.nnzRec) lif::k_gather_out<<<g, lif::THREADS, 0, st>>>(n, n.nnzRec, w, k.wOut);
+		const lif::AdjointPlan plan = relaxed || lif::capturing(st) ? lif::AdjointPlan() : lif::planAdjoint(n);
+		const int tw = plan.tw;
+		std::unique_ptr<lif::Turn> turn;
+		NEMO_CUDA(cudaMemsetAsync(k.barrier, 0, 8, st));
+		lif::Adjoint adj = {};
+		if(plan.parts) {
+			lif::k_out_count<<<g, lif::THREADS, 0, st>>>(n, plan.parts, plan.partRows, k.bucket);
+			lif::k_out_scan<<<plan.parts, 1024, 0, st>>>(n.N, k.bucket, k.total);
+			lif::k_out_fill<<<g, lif::THREADS, 0, st>>>(n, plan.parts, plan.partRows, tw * 4, k.bucket, k.total, w, k.entries);
+			adj.parts = plan.parts;
+			adj.partRows = plan.partRows;
+			adj.perGroup = plan.perGroup;
+			adj.sums = k.sums;
+			adj.bucket = k.bucket;
+			adj.total = k.total;
+			adj.entries = k.entries;
+			adj.uSeg = k.uSeg;
+			adj.guNext = k.guNext;
+			adj.guSeg = k.guSeg;
+			adj.dcounts = dcounts;
+			adj.barrier = k.barrier;
+			turn.reset(new lif::Turn(st));
+		} else if(n.nnzRec) {
+			lif::k_gather_out<<<g, lif::THREADS, 0, st>>>(n, n.nnzRec, w, k.wOut);
+		}
 		const int segments = (n.T + n.K - 1) / n.K;
 		const size_t units = size_t(n.N) + size_t(n.C);
 		const int L = lif::partSteps(std::min(n.K, n.T));
 		const unsigned gp = unsigned((n.N + lif::PART_WARPS - 1) / lif::PART_WARPS);
-		const size_t smemU = size_t(lif::PART_WARPS) * L * 32 * 4, smemW = smemU + lif::PART_WARPS * 32 * 4;
+		const size_t smemP = size_t(lif::PART_WARPS) * (size_t(L) * 32 + 32) * 4;
 		if(!relaxed) {
-			NEMO_CUDA(cudaFuncSetAttribute(lif::k_recompute, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemU)));
-			NEMO_CUDA(cudaFuncSetAttribute(lif::k_dw_events, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemW)));
+			NEMO_CUDA(cudaFuncSetAttribute(lif::k_recompute, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemP)));
+			NEMO_CUDA(cudaFuncSetAttribute(lif::k_dw_events, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemP)));
 		}
 		for(int sgi = segments - 1; sgi >= 0; --sgi) {
 			const int c0 = sgi * n.K, c1 = int(std::min<long>(n.T, long(c0) + n.K));
@@ -590,12 +1228,20 @@ nemo_b200_lif_backward(const nemo_b200_lif_net* net, const float* w, const uint3
 						in_bits, k.codes, k.cnt);
 				for(int y = 0; y < Y; ++y) {
 					const int t0 = c0 + y * L, t1 = std::min(c1, t0 + L);
-					lif::k_recompute<<<gp, lif::PART_WARPS * 32, smemU, st>>>(n, t0, t1, c0, L, w,
+					lif::k_recompute<<<gp, lif::PART_WARPS * 32, smemP, st>>>(n, tw, t0, t1, c0, L, w,
 							k.codes + size_t(y) * units * L * 32, k.cnt + size_t(y) * units, y ? k.v : ckpt, k.v, k.uSeg);
 				}
 			}
 			/* backwards through the segment */
-			for(int t = c1 - 1; t >= c0; --t) {
+			if(plan.parts) {
+				adj.c0 = c0;
+				adj.c1 = c1;
+				void* params[] = {&n, &adj};
+				NEMO_CUDA(cudaLaunchCooperativeKernel(lif::adjointKernel(tw), dim3(unsigned(plan.parts * plan.groups)),
+						dim3(unsigned(lif::ADJ_THREADS)), params, lif::ADJ_SMEM, st));
+				adj.barrierBase += unsigned(2 * (c1 - c0) - 1) * unsigned(plan.parts * plan.groups);
+			}
+			for(int t = c1 - 1; t >= c0 && !plan.parts; --t) {
 				const bool last = t == n.T - 1;
 				const float* next = t == c1 - 1 ? k.guNext : k.guSeg + size_t(t + 1 - c0) * NS;
 				lif::k_back<<<g, lif::THREADS, 0, st>>>(n, t, k.wOut, k.uSeg, c0, next, k.guSeg, dcounts, last);
@@ -605,11 +1251,11 @@ nemo_b200_lif_backward(const nemo_b200_lif_net* net, const float* w, const uint3
 			} else {
 				for(int y = 0; y < Y; ++y) {
 					const int t0 = c0 + y * L, t1 = std::min(c1, t0 + L);
-					lif::k_dw_events<<<gp, lif::PART_WARPS * 32, smemW, st>>>(n, t0, t1, c0, L, k.guSeg,
-							k.codes + size_t(y) * units * L * 32, k.cnt + size_t(y) * units, dw);
+					lif::k_dw_events<<<gp, lif::PART_WARPS * 32, smemP, st>>>(n, tw, t0, t1, c0, L, k.guSeg,
+							k.codes + size_t(y) * units * L * 32, k.cnt + size_t(y) * units, k.barrier + 1, dw);
 				}
 			}
-			NEMO_CUDA(cudaMemcpyAsync(k.guNext, k.guSeg, NS * 4, cudaMemcpyDeviceToDevice, st));
+			NEMO_CUDA(cudaMemcpyAsync(k.guNext, k.guSeg, size_t(n.N) * tw * 4, cudaMemcpyDeviceToDevice, st));
 		}
 		NEMO_CUDA(cudaGetLastError());
 	})
