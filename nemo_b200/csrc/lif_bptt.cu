@@ -937,6 +937,210 @@ k_adjoint(const __grid_constant__ Net n, const __grid_constant__ Adjoint a)
 	}
 }
 
+/* ---- the forward in one launch (spikes as bits) ----
+ *
+ * A step needs every neuron's spikes of the step before. One launch runs all
+ * steps with a grid barrier between them, where a launch per step costs the
+ * launch, the reload of every synapse from L2 (20 MB for 2.5e6) and a lane per
+ * trial that takes the synapses one by one. A block owns a contiguous range of
+ * neurons: their synapses, v and the step's spike words are in shared memory
+ * (synapses past its room are read from L2).
+ *
+ * A neuron is a warp. Lane L first has the spike word of synapse 31 - L of 32
+ * (bit b: trial b); the words are transposed (5 exchanges between lanes), after
+ * which lane b has the synapses that spike in trial b, the first one in the
+ * highest bit, and adds their weights in synapse order: as many turns as the
+ * busiest trial has spikes. What bounds a step is the shared-memory and
+ * exchange instructions and, with few neurons a block, their latency (a chain
+ * of about 1,000 clocks for 64 synapses): a warp whose block owns more neurons
+ * than warps takes two to four of them at once. */
+
+const int FWD_THREADS = 1024;
+const int FWD_WARPS = FWD_THREADS / 32;
+const size_t FWD_SMEM = 224 * 1024;
+
+struct Forward {
+	const float* w;
+	const uint32_t* inBits;
+	uint32_t* sBits;
+	float* vCkpt;
+	float* counts;
+	int perBlock;            /* neurons a block owns */
+	int cached;              /* synapses of a block in shared memory */
+	unsigned* barrier;       /* [0] arrivals, [1] error */
+};
+
+template<int NN>
+__global__ void __launch_bounds__(FWD_THREADS, 1)
+k_forward(const __grid_constant__ Net n, const __grid_constant__ Forward a)
+{
+	extern __shared__ __align__(128) char smem[];
+	__shared__ unsigned sCount[32];
+	const uint32_t lane = threadIdx.x & 31u;
+	const int warp = int(threadIdx.x >> 5);
+	const int units = n.N + n.C;
+	uint32_t* sWords = reinterpret_cast<uint32_t*>(smem);
+	float* sV = reinterpret_cast<float*>(sWords + (units + 31) / 32 * 32);
+	float* sW = sV + size_t(a.perBlock) * 32;
+	int* sPre = reinterpret_cast<int*>(sW + a.cached);
+	int* sRow = sPre + a.cached;   /* first synapse of each owned neuron, from the block's first one */
+	/* the transposition's exchange at distance d: keep the bits of keep[d],
+	 * take the others from the partner, rotated by turn[d] */
+	uint32_t keep[5], turn[5];
+	{
+		uint32_t m = 0x0000ffffu;
+#pragma unroll
+		for(int x = 0; x < 5; ++x) {
+			const uint32_t d = 16u >> x;
+			keep[x] = (lane & d) ? ~m : m;
+			turn[x] = (lane & d) ? 32u - d : d;
+			m ^= m << (d >> 1);
+		}
+	}
+
+	const int i0 = int(blockIdx.x) * a.perBlock;
+	const int own = max(0, min(a.perBlock, n.N - i0));
+	const int kFirst = own > 0 ? n.rowptr[i0] : 0;
+	const int kEnd = own > 0 ? n.rowptr[i0 + own] - kFirst : 0;
+	const int kCached = min(a.cached, kEnd);
+	for(int k = int(threadIdx.x); k < kCached; k += FWD_THREADS) {
+		sW[k] = a.w[kFirst + k];
+		sPre[k] = n.pre[kFirst + k];
+	}
+	for(int x = int(threadIdx.x); x < own * 32; x += FWD_THREADS) sV[x] = 0.0f;
+	for(int x = int(threadIdx.x); x <= own; x += FWD_THREADS) sRow[x] = own ? n.rowptr[i0 + x] - kFirst : 0;
+	if(threadIdx.x < 32) sCount[threadIdx.x] = 0u;
+
+	unsigned target = 0, spikes = 0;
+	for(int t = 0; t < n.T; ++t) {
+		/* the words this step's synapses deliver: the neurons' of the step
+		 * before (past the L1 cache: other blocks wrote them), the inputs' of
+		 * this step */
+		float* ckpt = t % n.K == 0 ? a.vCkpt + size_t(t / n.K) * n.N * 32 : nullptr;
+		const uint32_t* prev = a.sBits + size_t(t - 1) * n.N;
+		for(int p0 = int(threadIdx.x); p0 < n.N; p0 += 12 * FWD_THREADS) {
+			uint32_t x[12];
+#pragma unroll
+			for(int q = 0; q < 12; ++q) {
+				const int p = p0 + q * FWD_THREADS;
+				x[q] = t && p < n.N ? __ldcg(&prev[p]) : 0u;
+			}
+#pragma unroll
+			for(int q = 0; q < 12; ++q) {
+				const int p = p0 + q * FWD_THREADS;
+				if(p < n.N) sWords[p] = x[q];
+			}
+		}
+		for(int c = int(threadIdx.x); c < n.C; c += FWD_THREADS) sWords[n.N + c] = a.inBits[size_t(t) * n.C + c];
+		__syncthreads();
+		for(int l0 = warp * NN; l0 < own; l0 += FWD_WARPS * NN) {
+			/* NN neurons at once, C groups of 32 synapses of each (a neuron past
+			 * the block's last one: no synapses, nothing stored) */
+			const int C = NN == 1 ? 2 : 1;
+			float I[NN];
+			int k0[NN], k1[NN];
+			int most = 0;
+			bool near = true;
+#pragma unroll
+			for(int j = 0; j < NN; ++j) {
+				const bool in = l0 + j < own;
+				I[j] = 0.0f;
+				k0[j] = in ? sRow[l0 + j] : 0;
+				k1[j] = in ? sRow[l0 + j + 1] : 0;
+				most = max(most, k1[j] - k0[j]);
+				/* synapses in shared memory, or (some past the block's room)
+				 * all from L2 */
+				near = near && k1[j] <= kCached;
+			}
+			for(int base = 0; base < most; base += 32 * C) {
+				uint32_t word[NN][C];
+				float wk[NN][C];
+#pragma unroll
+				for(int j = 0; j < NN; ++j) {
+#pragma unroll
+					for(int c = 0; c < C; ++c) {
+						/* past the end: the neuron's last synapse (or the block's
+						 * first one), with no spikes */
+						const int k = k0[j] + base + c * 32 + 31 - int(lane);
+						const int kk = max(min(k, k1[j] - 1), 0);
+						const int p = near ? sPre[kk] : __ldg(&n.pre[kFirst + kk]);
+						wk[j][c] = near ? sW[kk] : __ldg(&a.w[kFirst + kk]);
+						word[j][c] = sWords[p] & (k < k1[j] ? FULL : 0u);
+					}
+				}
+#pragma unroll
+				for(int x = 0; x < 5; ++x) {
+#pragma unroll
+					for(int j = 0; j < NN; ++j) {
+#pragma unroll
+						for(int c = 0; c < C; ++c) {
+							const uint32_t y = __shfl_xor_sync(FULL, word[j][c], 16 >> x);
+							word[j][c] = (word[j][c] & keep[x]) | (__funnelshift_l(y, y, turn[x]) & ~keep[x]);
+						}
+					}
+				}
+#pragma unroll
+				for(int c = 0; c < C; ++c) {
+					unsigned spikesMost = 0;
+#pragma unroll
+					for(int j = 0; j < NN; ++j) spikesMost = max(spikesMost, unsigned(__popc(word[j][c])));
+					const unsigned turns = __reduce_max_sync(FULL, spikesMost);
+					/* two turns at once */
+					for(unsigned x = 0; x < turns; x += 2u) {
+#pragma unroll
+						for(int j = 0; j < NN; ++j) {
+							const uint32_t first = word[j][c];
+							const int q0 = 31 - __clz(int(first));
+							const uint32_t second = first & ~(1u << (q0 & 31));
+							const int q1 = 31 - __clz(int(second));
+							word[j][c] = second & ~(1u << (q1 & 31));
+							const float w0 = __shfl_sync(FULL, wk[j][c], q0), w1 = __shfl_sync(FULL, wk[j][c], q1);
+							if(first) I[j] = __fadd_rn(I[j], w0);
+							if(second) I[j] = __fadd_rn(I[j], w1);
+						}
+					}
+				}
+			}
+#pragma unroll
+			for(int j = 0; j < NN; ++j) {
+				if(l0 + j >= own) break;
+				const int l = l0 + j, i = i0 + l;
+				const float vPrev = sV[l * 32 + int(lane)];
+				if(ckpt) ckpt[size_t(i) * 32 + lane] = vPrev;
+				const float u = __fadd_rn(__fmul_rn(n.beta, vPrev), I[j]);
+				const bool s = lane < uint32_t(n.B) && u >= n.theta;
+				sV[l * 32 + int(lane)] = __fsub_rn(u, __fmul_rn(n.theta, s ? 1.0f : 0.0f));
+				const uint32_t out = __ballot_sync(FULL, s);
+				if(lane == 0) a.sBits[size_t(t) * n.N + i] = out;
+				spikes += s ? 1u : 0u;
+			}
+		}
+		if((t + 1) % n.binSteps == 0) {
+			/* whole numbers: the order does not matter */
+			if(spikes) atomicAdd(&sCount[lane], spikes);
+			spikes = 0;
+			__syncthreads();
+			if(threadIdx.x < uint32_t(n.B) && sCount[threadIdx.x]) {
+				atomicAdd(&a.counts[size_t(threadIdx.x) * (n.T / n.binSteps) + t / n.binSteps], float(sCount[threadIdx.x]));
+				sCount[threadIdx.x] = 0u;
+			}
+		}
+		if(t + 1 < n.T) {
+			if(gridDim.x == 1) {
+				__syncthreads();
+			} else {
+				target += gridDim.x;
+				gridArrive(a.barrier);
+				gridWait(a.barrier, target);
+			}
+		}
+	}
+	/* a barrier gave up: the counts become NaN */
+	if(threadIdx.x == 0 && *(volatile unsigned*) &a.barrier[1]) {
+		for(int x = 0; x < n.B * (n.T / n.binSteps); ++x) atomicAdd(&a.counts[x], __int_as_float(0x7fffffff));
+	}
+}
+
 static int
 grid(int N)
 {
@@ -1005,6 +1209,45 @@ planAdjoint(const Net& n)
 	p.groups = (n.N + per - 1) / per;
 	p.partRows = (n.N + parts - 1) / parts;
 	p.perGroup = per;
+	return p;
+}
+
+/* the forward with nn neurons a warp at once */
+static const void*
+forwardKernel(int nn)
+{
+	switch(nn) {
+		case 1: return (const void*) k_forward<1>;
+		case 2: return (const void*) k_forward<2>;
+		case 3: return (const void*) k_forward<3>;
+		default: return (const void*) k_forward<4>;
+	}
+}
+
+struct ForwardPlan {
+	int blocks = 0;   /* 0: step by step (k_step) */
+	int perBlock = 0, cached = 0;
+	const void* kernel = nullptr;
+};
+
+/* The forward in one launch, unless the spike words and v of a block do not
+ * fit its shared memory (past 45,000 neurons): eight neurons a block at least,
+ * a warp a neuron, a large network's neurons two to four a warp at once. */
+static ForwardPlan
+planForward(const Net& n)
+{
+	ForwardPlan p;
+	int most = residentBlocks(forwardKernel(1), FWD_THREADS, FWD_SMEM);
+	for(int nn = 2; nn <= 4; ++nn) most = std::min(most, residentBlocks(forwardKernel(nn), FWD_THREADS, FWD_SMEM));
+	if(most == 0) return p;
+	const int blocks = std::min(most, (n.N + 7) / 8);
+	const int per = (n.N + blocks - 1) / blocks;
+	const size_t fixed = (size_t(n.N) + size_t(n.C) + 31) / 32 * 128 + size_t(per) * 128 + (size_t(per) + 1) * 4;
+	if(fixed > FWD_SMEM) return p;
+	p.perBlock = per;
+	p.blocks = (n.N + per - 1) / per;
+	p.cached = int((FWD_SMEM - fixed) / 8);
+	p.kernel = forwardKernel(std::min(4, (per + FWD_WARPS - 1) / FWD_WARPS));
 	return p;
 }
 
@@ -1149,10 +1392,20 @@ nemo_b200_lif_forward(const nemo_b200_lif_net* net, const float* w, const uint32
 		cudaStream_t st = static_cast<cudaStream_t>(stream);
 		const LifWork k(n, work);
 		float* v = k.v;
-		NEMO_CUDA(cudaMemsetAsync(v, 0, size_t(n.N) * 32 * 4, st));
 		NEMO_CUDA(cudaMemsetAsync(counts, 0, size_t(n.B) * (n.T / n.binSteps) * 4, st));
 		const int g = lif::grid(n.N);
-		for(int t = 0; t < n.T; ++t) {
+		const lif::ForwardPlan plan = relaxed || lif::capturing(st) ? lif::ForwardPlan() : lif::planForward(n);
+		if(plan.blocks) {
+			NEMO_CUDA(cudaMemsetAsync(k.barrier, 0, 8, st));
+			lif::Forward f = {w, in_bits, s_bits, v_ckpt, counts, plan.perBlock, plan.cached, k.barrier};
+			std::unique_ptr<lif::Turn> turn;
+			if(plan.blocks > 1) turn.reset(new lif::Turn(st));
+			void* params[] = {&n, &f};
+			NEMO_CUDA(cudaLaunchCooperativeKernel(plan.kernel, dim3(unsigned(plan.blocks)),
+					dim3(unsigned(lif::FWD_THREADS)), params, lif::FWD_SMEM, st));
+		}
+		if(!plan.blocks) NEMO_CUDA(cudaMemsetAsync(v, 0, size_t(n.N) * 32 * 4, st));
+		for(int t = 0; t < n.T && !plan.blocks; ++t) {
 			if(relaxed) {
 				lif::k_step<true, false><<<g, lif::THREADS, 0, st>>>(n, t, w, in_bits, s_bits, s_float, v, v_ckpt,
 						counts, nullptr, 0);
