@@ -1758,6 +1758,35 @@ k_source_chunks(NetDev net, uint32_t* out)
 	}
 }
 
+/* reaches[b * blocks + x] = 1 for every bucket (source, block b) that is not
+ * empty, x the block that owns the source */
+__global__ void
+k_block_reaches(NetDev net, unsigned char* reaches)
+{
+	const uint32_t B = net.blocks;
+	const size_t total = size_t(B) * net.nDev;
+	for(size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < total; k += size_t(gridDim.x) * blockDim.x) {
+		if(net.segOff[k] == net.segOff[k + 1]) continue;
+		/* group g's buckets start at groupFirst[g] * nDev */
+		uint32_t g = 0;
+		while(size_t(net.groupFirst[g + 1]) * net.nDev <= k) ++g;
+		const uint32_t g0 = net.groupFirst[g], bg = net.groupFirst[g + 1] - g0;
+		const size_t rel = k - size_t(g0) * net.nDev;
+		const uint32_t src = uint32_t(rel / bg), b = g0 + uint32_t(rel % bg);
+		const uint32_t w = src / 32u;
+		if(w < net.warpBase || w >= net.warpBase + net.ownStart[B]) continue;   /* another shard's */
+		/* the last block that starts at or before the warp (blocks without
+		 * warps start where the next one does) */
+		uint32_t lo = 0, hi = B;
+		while(hi - lo > 1u) {
+			const uint32_t mid = (lo + hi) / 2u;
+			if(net.ownStart[mid] <= w - net.warpBase) lo = mid;
+			else hi = mid;
+		}
+		reaches[size_t(b) * B + lo] = 1;
+	}
+}
+
 /* hhDivConst against __fdiv_rn, divisors 20, 80 and 18, on every float with
  * magnitude at least 2^-100 (infinities included) and on both zeros */
 __global__ void
@@ -1996,6 +2025,12 @@ launchSourceChunks(const NetDev& net, uint32_t* srcChunk, void* stream)
 	const size_t total = (size_t(net.nDev) + 1) * net.groups;
 	const uint32_t blocks = uint32_t(std::min<size_t>((total + 255) / 256, size_t(smCount()) * 16));
 	k_source_chunks<<<std::max<uint32_t>(blocks, 1u), 256, 0, S(stream)>>>(net, srcChunk);
+}
+
+void
+launchBlockReaches(const NetDev& net, unsigned char* reaches, void* stream)
+{
+	k_block_reaches<<<smCount() * 8, 256, 0, S(stream)>>>(net, reaches);
 }
 
 void

@@ -376,6 +376,9 @@ void launchLibmEval(float* sinOut, float* logOut, const uint32_t* sinTab, const 
 void launchExpEval(uint32_t first, uint32_t n, float* out, const NetDev& net, void* stream);
 /* fill net.srcChunk from net.segOff (construction) */
 void launchSourceChunks(const NetDev& net, uint32_t* srcChunk, void* stream);
+/* reaches[b * blocks + x] = 1 where block x owns the source of a synapse of
+ * delay >= 2 into block b (construction; reaches zeroed by the caller) */
+void launchBlockReaches(const NetDev& net, unsigned char* reaches, void* stream);
 /* sharded simulation: the remote firing of cycle t (k_shard_inject) */
 void launchShardInject(const NetDev& net, uint64_t t, const uint32_t* allWords, uint32_t ownLo, uint32_t ownHi,
 		void* stream);

@@ -352,33 +352,10 @@ Simulation::construct(const Network& net, const Configuration& conf, const Shard
 	 * delay >= 2 synapses together stay within APPLY_GROUP_SYNAPSES (the
 	 * records one applyStdp launch rewrites, kept in L2) */
 	std::vector<uint32_t> groupFirst(1, 0), groupOf(B, 0);
-	/* and the blocks with such a synapse into each block (a shard's other
-	 * sources come with its remote list) */
-	std::vector<uint32_t> fromStart(1, 0), fromList;
 	{
 		std::vector<uint64_t> perBlock(size_t(B) + 1, 0);
-		std::vector<unsigned char> reaches(size_t(B) * B, 0);
 		for(size_t s = 0; s < S; ++s) {
-			if(net.dly[s] == 1) continue;
-			const uint32_t to = ownerOfWarp[dtgt[s] / 32 - warpLo];
-			perBlock[size_t(to) + 1]++;
-			const uint32_t w = dsrc[s] / 32;
-			if(w >= warpLo && w < m_shard.warpHi) reaches[size_t(to) * B + ownerOfWarp[w - warpLo]] = 1;
-		}
-		uint64_t buckets = 0;   /* (source, block) pairs that are looked up */
-		for(uint32_t b = 0; b < B; ++b) {
-			for(uint32_t x = 0; x < B; ++x) {
-				if(!reaches[size_t(b) * B + x]) continue;
-				fromList.push_back(x);
-				buckets += uint64_t(ownStart[x + 1] - ownStart[x]) * 32u;
-			}
-			fromStart.push_back(uint32_t(fromList.size()));
-		}
-		uint64_t records = 0;
-		for(uint32_t b = 0; b < B; ++b) records += perBlock[b + 1];
-		m_net.gatherSources = 32u;
-		while(m_net.gatherSources > 4u && records * m_net.gatherSources > uint64_t(GATHER_UNIT) * buckets) {
-			m_net.gatherSources /= 2u;
+			if(net.dly[s] != 1) perBlock[size_t(ownerOfWarp[dtgt[s] / 32 - warpLo]) + 1]++;
 		}
 		for(uint32_t b = 0; b < B; ++b) perBlock[b + 1] += perBlock[b];
 		for(uint32_t b = 0; b < B;) {
@@ -581,8 +558,36 @@ Simulation::construct(const Network& net, const Configuration& conf, const Shard
 		NEMO_CUDA(cudaGetLastError());
 		m_net.srcChunk = chunks;
 	}
-	m_net.fromStart = (const uint32_t*) put(fromStart.data(), fromStart.size() * 4);
-	m_net.fromList = (const uint32_t*) put(fromList.data(), fromList.size() * 4);
+	{
+		/* the blocks with a synapse of delay >= 2 into each block (a shard's
+		 * other sources come with its remote list), and the sources of a
+		 * gather unit by the average records of a (source, block) pair that is
+		 * looked up: from the device's segment offsets, since a pass over the
+		 * synapses here takes 10 ns each */
+		unsigned char* dReaches = (unsigned char*) alloc(size_t(B) * B);
+		launchBlockReaches(m_net, dReaches, m_stream);
+		NEMO_CUDA(cudaGetLastError());
+		std::vector<unsigned char> reaches(size_t(B) * B);
+		NEMO_CUDA(cudaMemcpyAsync(reaches.data(), dReaches, reaches.size(), cudaMemcpyDeviceToHost, stream));
+		NEMO_CUDA(cudaStreamSynchronize(stream));
+		std::vector<uint32_t> fromStart(1, 0), fromList;
+		uint64_t buckets = 0;
+		for(uint32_t b = 0; b < B; ++b) {
+			for(uint32_t x = 0; x < B; ++x) {
+				if(!reaches[size_t(b) * B + x]) continue;
+				fromList.push_back(x);
+				buckets += uint64_t(ownStart[x + 1] - ownStart[x]) * 32u;
+			}
+			fromStart.push_back(uint32_t(fromList.size()));
+		}
+		m_net.gatherSources = 32u;
+		while(m_net.gatherSources > 4u && d1Base * m_net.gatherSources > uint64_t(GATHER_UNIT) * buckets) {
+			m_net.gatherSources /= 2u;
+		}
+		m_net.fromStart = (const uint32_t*) put(fromStart.data(), fromStart.size() * 4);
+		m_net.fromList = (const uint32_t*) put(fromList.data(), fromList.size() * 4);
+		NEMO_CUDA(cudaStreamSynchronize(stream));   /* the lists are read from here */
+	}
 	m_net.outDegree = (const uint32_t*) put(outDegree.data(), outDegree.size() * 4);
 	m_net.d1Start = onDevice ? dev.d1Start : (const uint32_t*) put(d1Start.data(), d1Start.size() * 4);
 	m_net.d1Base = d1Base;
