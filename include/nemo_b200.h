@@ -343,7 +343,9 @@ nemo_status_t nemo_b200_expf_check(nemo_simulation_t sim, uint64_t* mismatches);
 /* Diagnostics: the Hodgkin-Huxley model's divisions of -(v + 65) by 20, 80
  * and 18 (an FMA-corrected product with the rounded reciprocal) against the
  * device's correctly rounded division, on every float of magnitude at least
- * 2^-100 and on the zeros; mismatches[q] per divisor (0 when they agree). */
+ * 2^-100 and on the zeros, and its branch-free divisions of the rates alpha_n,
+ * alpha_m and beta_h at every float voltage in their range; mismatches[q] per
+ * divisor, then per rate (added up; 0 when they agree). */
 nemo_status_t nemo_b200_hh_division_check(uint64_t mismatches[3]);
 
 /* The host-built table of inputs on which glibc expf rounds differently from

@@ -397,6 +397,53 @@ __device__ __forceinline__ float hhDivConst(float a, float d, float y)
 	return (r == 0.0f || !isfinite(q0)) ? q0 : q1;
 }
 
+/* num / den rounded to nearest without a branch, for operands whose magnitudes
+ * lie in [2^-40, 2^40) (hhDivInner): y = 1 / den from the hardware's
+ * approximation and one Newton step, q0 = RN(num y), the exact residual by
+ * FMA and one correction (P. Markstein, Computation of elementary functions
+ * on the IBM RISC System/6000 processor, 1990). Equal to __fdiv_rn for the
+ * three rates of every float voltage inside that range
+ * (nemo_b200_hh_division_check). */
+__device__ __forceinline__ float hhDiv(float num, float den)
+{
+	float y;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(den));
+	y = __fmaf_rn(__fmaf_rn(-den, y, 1.0f), y, y);
+	const float q0 = __fmul_rn(num, y);
+	return __fmaf_rn(__fmaf_rn(-q0, den, num), y, q0);
+}
+
+/* 0 when both magnitudes lie in [2^-40, 2^40) */
+__device__ __forceinline__ uint32_t hhDivOuter(float num, float den)
+{
+	const uint32_t lo = (127u - 40u) << 23, span = 80u << 23;
+	return uint32_t((__float_as_uint(num) & 0x7fffffffu) - lo >= span) | uint32_t((__float_as_uint(den) & 0x7fffffffu) - lo >= span);
+}
+
+/* a where the mask's bits are set, b elsewhere: a selection by lane that is
+ * an instruction, never a branch */
+__device__ __forceinline__ float hhSelect(uint32_t mask, float a, float b)
+{
+	return __uint_as_float((__float_as_uint(a) & mask) | (__float_as_uint(b) & ~mask));
+}
+
+/* The rate of lane role s (0..5 alpha_n, alpha_m, alpha_h, beta_n, beta_m,
+ * beta_h) at vr = v + 65, for every vr, by the general exponential and
+ * division (HH.cpp:92-98) */
+__device__ __forceinline__ float hhRate(const uint64_t* slots, uint32_t bits, uint32_t probe, uint32_t nearUnits, uint32_t s,
+		float vr)
+{
+	const float tenth = __fmul_rn(0.1f, vr);
+	const bool argDiv = s >= 2u && s <= 4u;
+	const float argA = s == 0u ? 1.0f : (s == 1u ? 2.5f : 3.0f);
+	const float argD = s == 2u ? 20.0f : (s == 3u ? 80.0f : 18.0f);
+	const float x = argDiv ? hhDivConst(-vr, argD, __fdiv_rn(1.0f, argD)) : __fsub_rn(argA, tenth);
+	const float e = libm::expf_match(x, slots, bits, probe, nearUnits);
+	if(argDiv) return __fmul_rn(s == 2u ? 0.07f : (s == 3u ? 0.125f : 4.0f), e);
+	const float num = s == 0u ? __fsub_rn(0.1f, __fmul_rn(0.01f, vr)) : (s == 1u ? __fsub_rn(2.5f, tenth) : 1.0f);
+	return __fdiv_rn(num, s == 5u ? __fadd_rn(e, 1.0f) : __fsub_rn(e, 1.0f));
+}
+
 /* Hodgkin-Huxley (src/nemo/cpu/plugins/HH.cpp:14-137): state v, n, m, h, dir;
  * no parameters. The currents act as conductances towards the reversal
  * potentials 0 and -70 mV. 999 Euler substeps of 0.001 ms ((int)(1/0.001f)
@@ -411,7 +458,18 @@ __device__ __forceinline__ float hhDivConst(float a, float d, float y)
  * shuffles; every lane then advances the same state with the same
  * operations. Called by all 32 lanes of a warp; `E`, `I` and the stimulus
  * are taken from the neuron's first lane. Returns the neuron's firing on all
- * its lanes. */
+ * its lanes.
+ *
+ * 999 substeps of one dependency chain with two or three such warps a
+ * scheduler: the latency of the chain and of every branch is the time. So a
+ * substep is straight-line code: lanes differ by constants and masks only (a
+ * branch on the lane's role costs about 75 clocks), the exponential goes
+ * without its range tests (|x| <= 80) and the division without its slow path.
+ * A warp with a lane outside those ranges, or with an exponential near a
+ * rounding midpoint (7% of the substeps), takes all its rates from hhRate.
+ * A substep of a warp takes 430 clocks where the code with branches took
+ * 1,300; 5,000 HH neurons among 50,000: 718 -> 360 us a cycle at rest, 873 ->
+ * 490 under stimulus. */
 __device__ __forceinline__ bool modelHH(const NetDev& net, const GroupDev& g, uint32_t i, float E, float I,
 		uint32_t stimWord, uint32_t cycle, uint32_t lane)
 {
@@ -441,32 +499,43 @@ __device__ __forceinline__ bool modelHH(const NetDev& net, const GroupDev& g, ui
 	const float RevE = 0.0f, RevI = -70.0f;
 	const int incMax = int(__fdiv_rn(1.0f, dt));
 	/* this lane's exponent: a - 0.1 (v + 65) for s = 0, 1, 5 (a = 1, 2.5,
-	 * 3), -(v + 65) / d for s = 2, 3, 4 (d = 20, 80, 18), none for 6, 7 */
-	const bool argDiv = s >= 2u && s <= 4u;
+	 * 3), -(v + 65) / d for s = 2, 3, 4 (d = 20, 80, 18), 0 for 6, 7 */
+	const uint32_t argDiv = s >= 2u && s <= 4u ? FULL : 0u, inUse = s < 6u ? FULL : 0u;
 	const float argA = s == 0u ? 1.0f : (s == 1u ? 2.5f : 3.0f);
 	const float argD = s == 2u ? 20.0f : (s == 3u ? 80.0f : 18.0f);
 	const float argY = __fdiv_rn(1.0f, argD);
-	/* this lane's rate: num / (e -+ 1) for s = 0, 1, 5, coef * e for 2, 3, 4 */
-	const bool rateDiv = s <= 1u || s == 5u;
+	/* this lane's rate: (a - b (v + 65)) / (e + c) for s = 0, 1, 5, coef * e
+	 * for 2, 3, 4 */
+	const uint32_t rateDiv = s <= 1u || s == 5u ? FULL : 0u;
+	const float numA = s == 0u ? 0.1f : (s == 1u ? 2.5f : 1.0f), numB = s == 0u ? 0.01f : (s == 1u ? 0.1f : 0.0f);
+	const float denC = s == 5u ? 1.0f : -1.0f;
 	const float rateCoef = s == 2u ? 0.07f : (s == 3u ? 0.125f : 4.0f);
-	const bool lookup = net.expProbe != 0u;
+	const uint32_t nearUnits = net.expProbe ? net.expNear : 0u;
+	const bool canFire = cycle >= 10u;
 	bool fired = false;
 	for(int t = 0; t < incMax; ++t) {
 		const float vr = __fadd_rn(v, 65.0f);
 		/* (RevI - v) / -1 is the exact negation */
 		const float I = __fadd_rn(__fadd_rn(__fmul_rn(Excit, __fsub_rn(RevE, v)),
 					__fmul_rn(Inhib, -__fsub_rn(RevI, v))), Exter);
-		const float tenth = __fmul_rn(0.1f, vr);
-		float x = argDiv ? hhDivConst(-vr, argD, argY) : __fsub_rn(argA, tenth);
-		x = s < 6u ? x : 0.0f;
-		const double cand = libm::exp_candidate_d(x);
-		float e = float(cand);
-		if(lookup && libm::exp_midpoint_units(cand) <= net.expNear) {
-			e = libm::exp_lookup(x, e, net.expSlots, net.expBits, net.expProbe);
+		/* hhDivConst without its tests: a residual of 0 leaves the quotient
+		 * (up to the sign of a 0, whose exponential is 1 either way), and one
+		 * that is not finite is out of range */
+		const float q0 = __fmul_rn(-vr, argY);
+		const float q1 = __fmaf_rn(__fmaf_rn(-q0, argD, -vr), argY, q0);
+		const float x = hhSelect(inUse, hhSelect(argDiv, q1, __fsub_rn(argA, __fmul_rn(0.1f, vr))), 0.0f);
+		const double cand = libm::exp_candidate_inner_d(x);
+		const float e = float(cand);
+		const float num = __fsub_rn(numA, __fmul_rn(numB, vr));
+		const float den = hhSelect(rateDiv, __fadd_rn(e, denC), 1.0f);
+		/* a neuron that is NaN (a rate of 0 / 0, which is not rare) stays so */
+		const bool number = vr == vr;
+		float rate = number ? hhSelect(rateDiv, hhDiv(num, den), __fmul_rn(rateCoef, e)) : vr;
+		const uint32_t general = uint32_t(libm::exp_midpoint_units_inner(cand) <= nearUnits)
+			| uint32_t(!(fabsf(x) <= 80.0f)) | hhDivOuter(num, den);
+		if(__any_sync(FULL, number && general != 0u)) {
+			rate = hhRate(net.expSlots, net.expBits, net.expProbe, net.expNear, s < 6u ? s : 2u, s < 6u ? vr : 0.0f);
 		}
-		const float num = s == 0u ? __fsub_rn(0.1f, __fmul_rn(0.01f, vr)) : (s == 1u ? __fsub_rn(2.5f, tenth) : 1.0f);
-		const float den = s == 5u ? __fadd_rn(e, 1.0f) : __fsub_rn(e, 1.0f);
-		const float rate = rateDiv ? __fdiv_rn(num, den) : __fmul_rn(rateCoef, e);
 		const float alphan = __shfl_sync(FULL, rate, lead + 0u);
 		const float alpham = __shfl_sync(FULL, rate, lead + 1u);
 		const float alphah = __shfl_sync(FULL, rate, lead + 2u);
@@ -485,11 +554,11 @@ __device__ __forceinline__ bool modelHH(const NetDev& net, const GroupDev& g, ui
 		/* division by C = 1 is exact */
 		const float newv = __fadd_rn(v, __fmul_rn(dt, __fadd_rn(-Ik, I)));
 		const float newDir = __fsub_rn(newv, v);
-		const float change = ((dir < 0.0f) | (newv < -45.0f)) ? 0.0f : newDir;
+		/* the change counts when the one before was not negative, above -45
+		 * mV; it is below -1e-9 (double) exactly when it is below the float
+		 * -1e-9, which lies on the side of 0 */
+		fired = fired | (canFire & !(dir < 0.0f) & !(newv < -45.0f) & (newDir < -1e-9f));
 		dir = newDir;
-		if(!fired && cycle >= 10u) {
-			fired = double(change) < -0.000000001;
-		}
 		v = newv;
 	}
 	fired = fired || stim;
@@ -501,6 +570,15 @@ __device__ __forceinline__ bool modelHH(const NetDev& net, const GroupDev& g, ui
 		S[4 * c + i] = dir;
 	}
 	return fired;
+}
+
+/* modelHH with registers of its own: the step kernel with the step-list and
+ * resident code has none to spare, and spilled the substep's
+ * (555 us a cycle of the mixed network against 495) */
+__device__ __noinline__ bool callHH(const NetDev& net, const GroupDev& g, uint32_t i, float E, float I, uint32_t stimWord,
+		uint32_t cycle, uint32_t lane)
+{
+	return modelHH(net, g, i, E, I, stimWord, cycle, lane);
 }
 
 /* PoissonSource (src/nemo/cpu/plugins/PoissonSource.cpp:21-29). The
@@ -827,13 +905,14 @@ __device__ __forceinline__ void writeStepList(const NetDev& net, uint32_t* hostW
 /* k_cycles: see kernels.hpp for the phase structure. HOST: the launch may
  * write a step list to host memory or stay resident (CycleArgs::hostWords,
  * cmd); launches that do neither use the instantiation without that code,
- * which leaves the rest more registers. The forward regions and
+ * which leaves the rest more registers. HH: the network has Hodgkin-Huxley
+ * neurons; the others run without that model's code for the same reason. The forward regions and
  * the reverse-matrix arrays are streamed with evict-first loads and stores
  * (__ldcs / __stcs), so that they do not push the randomly read firing
  * history, segment offsets and noise tables out of L2. SMEM: the owned current
  * slots live in dynamic shared memory as int32 E/I pairs,
  * sAcc[slot * ownN + local]; otherwise every access goes to net.acc. */
-template<bool SMEM, unsigned T, bool HOST>
+template<bool SMEM, unsigned T, bool HOST, bool HH>
 __global__ void __launch_bounds__(T, 1)
 k_cycles(const __grid_constant__ CycleArgs A)
 {
@@ -1025,9 +1104,11 @@ k_cycles(const __grid_constant__ CycleArgs A)
 				const float E = wfxToFloat(e, net.fbits);
 				const float I = wfxToFloat(in, net.fbits);
 				bool fired = false;
-				if(G.kind == 3) {   /* MODEL_HH */
+				if(HH && G.kind == 3) {   /* MODEL_HH */
 					/* all lanes: eight per neuron */
-					fired = modelHH(net, G, i, E, I, stimWord, t - G.timerBase, lane) && valid;
+					fired = HOST ? callHH(net, G, i, E, I, stimWord, t - G.timerBase, lane)
+						: modelHH(net, G, i, E, I, stimWord, t - G.timerBase, lane);
+					fired = fired && valid;
 				} else if(valid) {
 					const bool stim = (stimWord >> lane) & 1u;
 					switch(G.kind) {
@@ -1788,7 +1869,9 @@ k_block_reaches(NetDev net, unsigned char* reaches)
 }
 
 /* hhDivConst against __fdiv_rn, divisors 20, 80 and 18, on every float with
- * magnitude at least 2^-100 (infinities included) and on both zeros */
+ * magnitude at least 2^-100 (infinities included) and on both zeros; hhDiv
+ * against __fdiv_rn for the rates alpha_n, alpha_m and beta_h at every float
+ * voltage */
 __global__ void
 k_hh_div_check(unsigned long long* bad)
 {
@@ -1797,6 +1880,22 @@ k_hh_div_check(unsigned long long* bad)
 	const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
 	for(uint64_t u = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; u < (uint64_t(1) << 32); u += stride) {
 		const float a = libm::u2f(uint32_t(u));
+		/* the rates at the voltage u: inside hhDiv's range every quotient is
+		 * __fdiv_rn's; glibc's exponential is the candidate or a neighbour */
+		const float vr = __fadd_rn(a, 65.0f);
+		const float tenth = __fmul_rn(0.1f, vr);
+#pragma unroll
+		for(int q = 0; q < 3; ++q) {
+			const float x = __fsub_rn(q == 0 ? 1.0f : (q == 1 ? 2.5f : 3.0f), tenth);
+			if(!(fabsf(x) <= 80.0f)) continue;
+			const float num = q == 0 ? __fsub_rn(0.1f, __fmul_rn(0.01f, vr)) : (q == 1 ? x : 1.0f);
+			const float e = float(libm::exp_candidate_inner_d(x));
+#pragma unroll
+			for(int o = -1; o <= 1; ++o) {
+				const float den = __fadd_rn(libm::u2f(libm::f2u(e) + uint32_t(o)), q == 2 ? 1.0f : -1.0f);
+				if(!hhDivOuter(num, den) && libm::f2u(hhDiv(num, den)) != libm::f2u(__fdiv_rn(num, den))) nb[q]++;
+			}
+		}
 		if(!(fabsf(a) >= 0x1p-100f) && a != 0.0f) continue;   /* NaN and tiny magnitudes */
 #pragma unroll
 		for(int q = 0; q < 3; ++q) {
@@ -1872,13 +1971,36 @@ launchStimulusScratch(const NetDev& net, const uint32_t* scratch, uint32_t nf, u
 	k_stimulus_scratch<<<blocks, 256, 0, S(stream)>>>(net, scratch, nf, ni);
 }
 
+template<bool SMEM, bool HOST, bool HH>
+static const void*
+cyclesKernelT(uint32_t threads)
+{
+	switch(threads) {
+		case 256: return (const void*) k_cycles<SMEM, 256, HOST, HH>;
+		case 512: return (const void*) k_cycles<SMEM, 512, HOST, HH>;
+		default: return (const void*) k_cycles<SMEM, 1024, HOST, HH>;
+	}
+}
+
+/* the instantiation of the step kernel */
+static const void*
+cyclesKernel(bool smem, uint32_t threads, bool host, bool hh)
+{
+	if(smem) {
+		return host ? (hh ? cyclesKernelT<true, true, true>(threads) : cyclesKernelT<true, true, false>(threads))
+			: (hh ? cyclesKernelT<true, false, true>(threads) : cyclesKernelT<true, false, false>(threads));
+	}
+	return host ? (hh ? cyclesKernelT<false, true, true>(threads) : cyclesKernelT<false, true, false>(threads))
+		: (hh ? cyclesKernelT<false, false, true>(threads) : cyclesKernelT<false, false, false>(threads));
+}
+
 /* The step kernel's plan: one 1024-thread block per SM (its registers allow
  * no more) and no block without neurons; the neuron warps split into
  * contiguous ranges of about equal summed update cost (block b starts at the
  * first warp whose cost prefix reaches b / B of the total); the owned
  * current slots go to shared memory when they are int32 and fit. */
 void
-cyclesPlan(const std::vector<uint32_t>& warpCost, uint32_t slots, bool acc32, uint32_t* blocks,
+cyclesPlan(const std::vector<uint32_t>& warpCost, uint32_t slots, bool acc32, bool hh, uint32_t* blocks,
 		std::vector<uint32_t>* ownStart, uint32_t* ownWarps, bool* smemAcc)
 {
 	const uint32_t totalWarps = uint32_t(warpCost.size());
@@ -1902,65 +2024,19 @@ cyclesPlan(const std::vector<uint32_t>& warpCost, uint32_t slots, bool acc32, ui
 	const bool smem = acc32 && bytes <= SMEM_ACC_LIMIT;
 	/* the attribute is per device and shared by all simulations: set it to
 	 * the largest size any of them uses */
-	cudaFuncSetAttribute(k_cycles<true, 1024, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_ACC_LIMIT));
-	cudaFuncSetAttribute(k_cycles<true, 512, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_ACC_LIMIT));
-	cudaFuncSetAttribute(k_cycles<true, 256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_ACC_LIMIT));
-	cudaFuncSetAttribute(k_cycles<true, 1024, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_ACC_LIMIT));
-	cudaFuncSetAttribute(k_cycles<true, 512, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_ACC_LIMIT));
-	cudaFuncSetAttribute(k_cycles<true, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_ACC_LIMIT));
 	int perSm = 0, perSmHost = 0;
-	if(smem) {
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_cycles<true, 1024, false>, 1024, size_t(bytes));
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSmHost, k_cycles<true, 1024, true>, 1024, size_t(bytes));
-	} else {
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_cycles<false, 1024, false>, 1024, 0);
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSmHost, k_cycles<false, 1024, true>, 1024, 0);
+	for(int v = 0; smem && v < 12; ++v) {
+		const uint32_t threads = v % 3 == 0 ? 1024u : (v % 3 == 1 ? 512u : 256u);
+		cudaFuncSetAttribute(cyclesKernel(true, threads, v / 3 % 2, v / 6), cudaFuncAttributeMaxDynamicSharedMemorySize,
+				int(SMEM_ACC_LIMIT));
 	}
+	const size_t dyn = smem ? size_t(bytes) : 0;
+	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, cyclesKernel(smem, 1024, false, hh), 1024, dyn);
+	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSmHost, cyclesKernel(smem, 1024, true, hh), 1024, dyn);
 	perSm = std::min(perSm, perSmHost);
 	*blocks = perSm >= 1 ? B : 0u;
 	*ownWarps = most;
 	*smemAcc = smem;
-}
-
-template<bool SMEM, bool HOST>
-static cudaError_t
-launchCyclesH(const CycleArgs& args, void** params, size_t bytes, cudaStream_t stream)
-{
-	const NetDev& net = args.net;
-	if(args.cycles <= 1u && (args.carry & 2u) && args.cmd == nullptr) {
-		/* one update phase and no grid barrier: the blocks never wait for one
-		 * another, so they need not be co-resident */
-		switch(net.threads) {
-			case 256:
-				return cudaLaunchKernel((const void*) k_cycles<SMEM, 256, HOST>, dim3(net.blocks), dim3(256), params,
-						bytes, stream);
-			case 512:
-				return cudaLaunchKernel((const void*) k_cycles<SMEM, 512, HOST>, dim3(net.blocks), dim3(512), params,
-						bytes, stream);
-			default:
-				return cudaLaunchKernel((const void*) k_cycles<SMEM, 1024, HOST>, dim3(net.blocks), dim3(1024), params,
-						bytes, stream);
-		}
-	}
-	switch(net.threads) {
-		case 256:
-			return cudaLaunchCooperativeKernel((const void*) k_cycles<SMEM, 256, HOST>, dim3(net.blocks), dim3(256),
-					params, bytes, stream);
-		case 512:
-			return cudaLaunchCooperativeKernel((const void*) k_cycles<SMEM, 512, HOST>, dim3(net.blocks), dim3(512),
-					params, bytes, stream);
-		default:
-			return cudaLaunchCooperativeKernel((const void*) k_cycles<SMEM, 1024, HOST>, dim3(net.blocks), dim3(1024),
-					params, bytes, stream);
-	}
-}
-
-template<bool SMEM>
-static cudaError_t
-launchCyclesT(const CycleArgs& args, void** params, size_t bytes, cudaStream_t stream)
-{
-	if(args.hostWords || args.cmd) return launchCyclesH<SMEM, true>(args, params, bytes, stream);
-	return launchCyclesH<SMEM, false>(args, params, bytes, stream);
 }
 
 void
@@ -1968,11 +2044,18 @@ launchCycles(const CycleArgs& args, void* stream)
 {
 	void* params[] = {const_cast<CycleArgs*>(&args)};
 	const NetDev& net = args.net;
-	if(net.smemAcc && !args.globalAcc) {
-		const size_t bytes = size_t(net.slots) * net.ownWarps * 32u * 8u;
-		launchCyclesT<true>(args, params, bytes, S(stream));
+	const bool smem = net.smemAcc && !args.globalAcc;
+	bool hh = false;
+	for(int g = 0; g < args.ngroups; ++g) hh = hh || args.groups[g].kind == 3;   /* MODEL_HH */
+	const void* kernel = cyclesKernel(smem, net.threads, args.hostWords || args.cmd, hh);
+	const size_t bytes = smem ? size_t(net.slots) * net.ownWarps * 32u * 8u : 0;
+	const uint32_t threads = net.threads == 256u || net.threads == 512u ? net.threads : 1024u;
+	if(args.cycles <= 1u && (args.carry & 2u) && args.cmd == nullptr) {
+		/* one update phase and no grid barrier: the blocks never wait for one
+		 * another, so they need not be co-resident */
+		cudaLaunchKernel(kernel, dim3(net.blocks), dim3(threads), params, bytes, S(stream));
 	} else {
-		launchCyclesT<false>(args, params, 0, S(stream));
+		cudaLaunchCooperativeKernel(kernel, dim3(net.blocks), dim3(threads), params, bytes, S(stream));
 	}
 }
 

@@ -361,8 +361,8 @@ void launchCycles(const CycleArgs& args, void* stream);
  * the neuron warps over its blocks: contiguous ranges of about equal summed
  * cost (warpCost[w]: the update cost of warp w), ownStart[blocks + 1]; the
  * most warps a block owns, and whether the owned current slots fit in shared
- * memory. */
-void cyclesPlan(const std::vector<uint32_t>& warpCost, uint32_t slots, bool acc32, uint32_t* blocks,
+ * memory. hh: the network has Hodgkin-Huxley neurons. */
+void cyclesPlan(const std::vector<uint32_t>& warpCost, uint32_t slots, bool acc32, bool hh, uint32_t* blocks,
 		std::vector<uint32_t>* ownStart, uint32_t* ownWarps, bool* smemAcc);
 /* applyStdp over target groups [groupTargets[g], groupTargets[g+1]), one
  * launch per group (groups of owner blocks, see APPLY_GROUP_SYNAPSES);

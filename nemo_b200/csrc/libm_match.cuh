@@ -207,10 +207,11 @@ LIBM_HD float log_candidate(float y) { return float(log_candidate_d(y)); }
  * k = round(x / ln2) by adding 1.5 * 2^52 (the fused x * (1/ln2) + 1.5 * 2^52
  * rounds once, to a double whose last place is 1), r = x - k ln2 with the
  * Cody-Waite split of ln2 (|r| <= 0.3466), e^r by its Taylor series to degree
- * 11 (truncation below 7e-15 relative) in Estrin's scheme, scaled by 2^k.
- * Beyond the float range: 0 below -104, infinity above 89; NaN stays NaN.
- * The result is branch-free, so that several evaluations interleave. */
-LIBM_HD double exp_candidate_d(float xf) {
+ * 11 (truncation below 7e-15 relative) in Estrin's scheme (exp_reduced_d: e^r
+ * and k), scaled by 2^k. Beyond the float range: 0 below -104, infinity above
+ * 89; NaN stays NaN. The result is branch-free, so that several evaluations
+ * interleave. */
+LIBM_HD double exp_reduced_d(float xf, uint32_t* kOut) {
 	const double ln2_hi = 6.93147180369123816490e-01;  /* 0x3FE62E42FEE00000 */
 	const double ln2_lo = 1.90821492927058770002e-10;
 	const double shift = 6755399441055744.0;            /* 1.5 * 2^52 */
@@ -232,12 +233,34 @@ LIBM_HD double exp_candidate_d(float xf) {
 	const double b1 = D_FMA(r2, a3, a2);
 	const double b2 = D_FMA(r2, a5, a4);
 	const double r8 = D_MUL(r4, r4);
-	const double p = D_FMA(r8, b2, D_FMA(r4, b1, b0));
+	*kOut = k;
+	return D_FMA(r8, b2, D_FMA(r4, b1, b0));
+}
+
+/* The candidate for |x| <= 80, where 2^k is applied as an addition to the
+ * exponent field: e^r is in [0.70, 1.42], so that the result is a normal
+ * number and the product with 2^k is that sum exactly. */
+LIBM_HD double exp_candidate_inner_d(float xf) {
+	uint32_t k;
+	const double p = exp_reduced_d(xf, &k);
+	return u2d(d2u(p) + (uint64_t(k) << 52));
+}
+
+LIBM_HD double exp_candidate_d(float xf) {
+	uint32_t k;
+	const double x = double(xf);
+	const double p = exp_reduced_d(xf, &k);
 	/* 2^k is a normal double for every k the range [-104, 89] gives */
 	double res = D_MUL(p, u2d(uint64_t((1023u + k) & 0x7FFu) << 52));
 	res = xf > 89.0f ? u2d(0x7FF0000000000000ull) : res;
 	res = xf < -104.0f ? 0.0 : res;
 	return xf == xf ? res : x;
+}
+
+/* exp_midpoint_units of a candidate in the float normal range */
+LIBM_HD uint32_t exp_midpoint_units_inner(double c) {
+	const int32_t d = int32_t(uint32_t(d2u(c)) & 0x1FFFFFFFu) - 0x10000000;
+	return uint32_t(d < 0 ? -d : d);
 }
 
 /* How close the double candidate c lies to a float rounding midpoint: the
@@ -250,8 +273,7 @@ LIBM_HD uint32_t exp_midpoint_units(double c) {
 	const uint64_t b = d2u(c);
 	const uint32_t e = uint32_t(b >> 52) & 0x7FFu;
 	if(e < 897u || e > 1150u) return 0u;
-	const int32_t d = int32_t(uint32_t(b) & 0x1FFFFFFFu) - 0x10000000;
-	return uint32_t(d < 0 ? -d : d);
+	return exp_midpoint_units_inner(c);
 }
 
 /* The exception table as an open-addressing hash: 2^bits slots of

@@ -319,19 +319,24 @@ Simulation::construct(const Network& net, const Configuration& conf, const Shard
 	}
 
 	/* update cost per owned warp: an HH warp (999 substeps of six exponentials
-	 * over eight lanes per neuron) counts 2.5 times another model's, so that
+	 * over eight lanes per neuron) counts 3 times another model's, so that
 	 * HH warps spread over more blocks while no block owns more warps than it
-	 * has update warps in a mixed network of a few HH neurons per ten others */
+	 * has update warps in a mixed network of a few HH neurons per ten others
+	 * (1,250 HH warps beside 1,407 others: at most 12 a block, three a
+	 * scheduler; with 2.5 times some blocks own 13 and a scheduler has four,
+	 * 716 clocks a substep against 587) */
 	std::vector<uint32_t> warpCost(m_shard.warpHi - warpLo, 2u);
+	bool hh = false;
 	for(const Group& g : m_groups) {
 		if(g.type.kind != MODEL_HH) continue;
+		hh = true;
 		const uint32_t w0 = g.devBase / 32, w1 = uint32_t((uint64_t(g.devBase) + (uint64_t(g.count) << g.shift) + 31) / 32);
-		for(uint32_t w = std::max(w0, warpLo); w < std::min(w1, m_shard.warpHi); ++w) warpCost[w - warpLo] = 5u;
+		for(uint32_t w = std::max(w0, warpLo); w < std::min(w1, m_shard.warpHi); ++w) warpCost[w - warpLo] = 6u;
 	}
 	std::vector<uint32_t> ownStart;
 	uint32_t ownWarps = 0;
 	bool smemAcc = false;
-	cyclesPlan(warpCost, slots, acc32, &m_blocks, &ownStart, &ownWarps, &smemAcc);
+	cyclesPlan(warpCost, slots, acc32, hh, &m_blocks, &ownStart, &ownWarps, &smemAcc);
 	/* owner block of each owned warp */
 	std::vector<uint32_t> ownerOfWarp(warpCost.size(), 0);
 	for(uint32_t b = 0; b + 1 < ownStart.size(); ++b) {
