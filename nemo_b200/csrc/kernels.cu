@@ -836,6 +836,30 @@ __device__ __forceinline__ bool residentWait(const CycleArgs& A, uint32_t seq, u
 	return ok != 0;
 }
 
+/* Wait until every block of a resident launch has arrived after its update
+ * (thread 0; false when it gives up after timeoutNs). */
+__device__ __forceinline__ bool residentArrived(unsigned* count, unsigned all, unsigned long long timeoutNs)
+{
+	__shared__ int ok;
+	if(threadIdx.x == 0) {
+		const size_t addr = __cvta_generic_to_global(count);
+		const unsigned long long start = globalTimer();
+		int good = 1;
+		for(uint32_t spins = 0;; ++spins) {
+			uint32_t v;
+			asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(addr) : "memory");
+			if(int(v - all) >= 0) break;
+			if((spins & 255u) == 255u && globalTimer() - start > timeoutNs) {
+				good = 0;
+				break;
+			}
+		}
+		ok = good;
+	}
+	__syncthreads();
+	return ok != 0;
+}
+
 /* Add one forward-matrix record into current slot `slot` of its target
  * (E for w >= 0, else I), in shared memory or in net.acc */
 template<bool SMEM>
@@ -978,18 +1002,27 @@ k_cycles(const __grid_constant__ CycleArgs A)
 	 * gathering waits for the next launch, and nothing follows that phase,
 	 * so it needs no grid barrier after it (a one-cycle step has none at
 	 * all and runs as an ordinary launch) */
-	/* resident stepping (CycleArgs::cmd): one update phase per command until
-	 * an exit command or the idle limit; the last cycle stays pending */
+	/* resident stepping (CycleArgs::cmd): an update phase and its gather phase
+	 * per command until an exit command or the idle limit; nothing stays
+	 * pending but the delay-1 arrivals in the inbox */
 	const bool resident = HOST && A.cmd != nullptr;
 	const bool lastPending = resident || (A.carry & 2u) != 0u;
 	const uint32_t phases = resident ? 0xffffffffu : A.cycles + (lastPending ? 0u : 1u);
+	/* a resident launch's count of block arrivals after the updates when it
+	 * started */
+	const unsigned doneBase = HOST ? *(volatile unsigned*) &net.barrier[5] : 0u;
 	const uint32_t barriers = lastPending && A.cycles ? A.cycles - 1u : A.cycles;
 	uint32_t passed = 0;   /* grid barriers passed */
-	uint32_t k = 0;
-	for(; k < phases; ++k) {
-		const uint64_t t64 = first + k;
+	uint32_t k = 0;        /* the update (resident: the command), counted from the launch's start */
+	for(uint32_t phase = 0; phase < phases; ++phase) {
+		/* resident stepping: two phases a command, the update (after which the
+		 * host has its step list) and then the gathering and learning of the
+		 * same cycle, while the host prepares the next command */
+		k = resident ? phase >> 1 : phase;
+		const bool after = resident && (phase & 1u);
+		const uint64_t t64 = first + (resident ? (phase + 1u) >> 1 : phase);
 		const uint32_t t = uint32_t(t64);
-		const bool doUpdate = resident || k < A.cycles;
+		const bool doUpdate = resident ? !after : k < A.cycles;
 		/* this phase's stimulus: the launch's own (first phase), or the
 		 * command block 0 copied before the last grid barrier */
 		uint32_t stNf = 0u, stNi = 0u;
@@ -1002,7 +1035,7 @@ k_cycles(const __grid_constant__ CycleArgs A)
 			stF = A.inlineF;
 			stI = A.inlineI;
 			stC = A.inlineCur;
-		} else if(resident) {
+		} else if(resident && doUpdate) {
 			const ResidentCmd* c = A.bcast + (k & 1u);
 			stNf = c->nf;
 			stNi = c->ni;
@@ -1010,7 +1043,8 @@ k_cycles(const __grid_constant__ CycleArgs A)
 			stI = c->i;
 			stC = c->cur;
 		}
-		const bool doPrev = k > 0 || (A.carry & 1u);     /* gather and learn for cycle t-1 */
+		/* gather and learn for cycle t-1 */
+		const bool doPrev = resident ? after || (phase == 0 && (A.carry & 1u)) : k > 0 || (A.carry & 1u);
 		const uint32_t slotT = uint32_t(t64 % net.slots);
 
 		if(tid == 0) {
@@ -1280,7 +1314,7 @@ k_cycles(const __grid_constant__ CycleArgs A)
 			const uint32_t Sb = P > b ? (P - b + B - 1u) / B : 0u;
 			/* units [G, G + NW): the next cycle's noise of one owned neuron
 			 * warp each (from the second phase of a launch on) */
-			const uint32_t NW = (k + 1u < A.cycles || (resident && k > 0u)) ? myWarps : 0u;
+			const uint32_t NW = (resident ? after && k > 0u : k + 1u < A.cycles) ? myWarps : 0u;
 			const uint32_t units = G + NW + Sb;
 			const uint32_t* flist = net.firedList + par * listStride;
 			const uint2* plist = net.postList + par * postParity;
@@ -1400,9 +1434,9 @@ k_cycles(const __grid_constant__ CycleArgs A)
 					const uint32_t i = n - Gr.devBase;
 					if(Gr.kind == 0 && i < Gr.count) {
 						if(resident) {
-							/* from the state this cycle's update advances the
-							 * generator to */
-							drawNoiseAhead(net, Gr, i, n, net.rngAhead[size_t(t & 1u) * nDev + n], (t + 1u) & 1u);
+							/* cycle t's, from the state the update of cycle t - 1
+							 * advanced the generator to */
+							drawNoiseAhead(net, Gr, i, n, net.rngAhead[size_t((t - 1u) & 1u) * nDev + n], t & 1u);
 						} else {
 							net.noise[((t + 1u) & 1u) * nDev + n] = drawNoise(net, Gr, i);
 						}
@@ -1484,17 +1518,19 @@ k_cycles(const __grid_constant__ CycleArgs A)
 		}
 		if(trace && tid == 0) trace[3] = globalTimer();
 		if(HOST && A.hostWords && doUpdate) {
-			/* the step's list, by the block whose update arrives last */
+			/* the step's list, by the block whose update arrives last: the
+			 * count starts again for the next step (which the host starts after
+			 * this one's list), or in a resident launch goes on */
+			const unsigned all = doneBase + (k + 1u) * B;
 			if(tid == 0) {
 				__threadfence();
-				sLast = atomicAdd(&net.barrier[3], 1u) == B - 1u;
-				if(sLast) {
-					/* every block has arrived: the count starts again for
-					 * the next step, which the host starts after this one's
-					 * list */
-					*(volatile unsigned*) &net.barrier[3] = 0u;
-					__threadfence();
+				if(resident) {
+					sLast = atomicAdd(&net.barrier[4], 1u) + 1u == all;
+				} else {
+					sLast = atomicAdd(&net.barrier[3], 1u) == B - 1u;
+					if(sLast) *(volatile unsigned*) &net.barrier[3] = 0u;
 				}
+				if(sLast) __threadfence();
 			}
 			__syncthreads();
 			if(sLast) {
@@ -1504,8 +1540,13 @@ k_cycles(const __grid_constant__ CycleArgs A)
 					*(volatile uint32_t*) &A.doneWords[0] = A.firstSeq + k;
 				}
 			}
+			/* a resident launch gathers the cycle once every block has updated */
+			if(resident && !residentArrived(&net.barrier[4], all, A.timeoutNs)) {
+				if(tid == 0) A.hostWords[0] = 1u;
+				return;
+			}
 		}
-		if(resident) {
+		if(after) {
 			/* block 0 waits for the next command and hands it to every
 			 * block */
 			const uint32_t seqK = A.firstSeq + k;
@@ -1516,7 +1557,7 @@ k_cycles(const __grid_constant__ CycleArgs A)
 				return;
 			}
 			if(*(volatile const uint32_t*) &A.bcast[(k + 1u) & 1u].op != RESIDENT_STEP) break;
-		} else if(k < barriers) {
+		} else if(!resident && k < barriers) {
 			if(!gridSync(net.barrier, barBase + (k + 1u) * B, A.timeoutNs)) {
 				if(HOST && A.hostWords && tid == 0) A.hostWords[0] = 1u;
 				return;
@@ -1567,6 +1608,7 @@ k_cycles(const __grid_constant__ CycleArgs A)
 		if(resident) {
 			/* the commands up to firstSeq + k ran; the host waits for the
 			 * stream before anything else */
+			*(volatile unsigned*) &net.barrier[5] = doneBase + (k + 1u) * B;
 			__threadfence_system();
 			*(volatile uint32_t*) A.exitInfo = ((A.firstSeq + k) << 1) | 1u;
 		}

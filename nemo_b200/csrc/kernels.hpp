@@ -187,7 +187,8 @@ struct NetDev {
 	/* grid barrier: [0] arrivals since the simulation was created (every
 	 * block adds 1 at every barrier), [1] the arrival count when the current
 	 * launch started (written by block 0 at the end of each launch), [2]
-	 * error (timeout) */
+	 * error (timeout), [3] arrivals of a one-cycle step's blocks at its list,
+	 * [4] and [5] as [0] and [1] for the updates of resident launches */
 	unsigned* barrier;
 };
 
@@ -291,18 +292,21 @@ struct CycleArgs {
 	/* when set, the first cycle is read from here instead of firstCycle and
 	 * advanced by the launch (launches replayed from a CUDA graph) */
 	uint64_t* cycleCounter;
-	/* resident stepping: when cmd is set, the launch runs one update phase
-	 * per command instead of `cycles` phases. The first command (seq
-	 * firstSeq) is this launch's inline stimulus; after each phase the block
-	 * that writes the step list writes the command's seq into doneWords[0]
-	 * (mapped host memory) after it, and block 0 waits for command seq + 1 in
-	 * *cmd (mapped host memory) for at most idleNs and copies it to
-	 * bcast[(phase + 1) & 1] (device), where the other blocks wait for it.
-	 * The host issues a command only after the done word has come, which
-	 * follows every block's phase, so no grid barrier separates the phases. An exit
-	 * command, or no command within idleNs, ends the launch, which leaves its
-	 * last cycle pending (as carry bit 1) and writes exitInfo = (last seq done
-	 * << 1) | 1 (mapped host memory). */
+	/* resident stepping: when cmd is set, the launch runs two phases per
+	 * command instead of `cycles` phases. The first command (seq firstSeq) is
+	 * this launch's inline stimulus. The update phase ends with the step list
+	 * and the command's seq in doneWords[0] (mapped host memory), written by the
+	 * block whose update arrives last; once every block has arrived
+	 * (NetDev::barrier[4]) the second phase gathers and learns for the same
+	 * cycle and draws the next one's noise, while the host has its list and
+	 * prepares the next command. Block 0 then waits for command seq + 1 in *cmd
+	 * (mapped host memory) for at most idleNs and copies it to
+	 * bcast[(update + 1) & 1] (device), where the other blocks wait for it. A
+	 * block may be in the next update while another still gathers: what a
+	 * gather reads is kept by cycle parity, and no block gathers the next cycle
+	 * before all have updated it. An exit command, or no command within idleNs,
+	 * ends the launch with nothing pending but the inbox, and writes exitInfo =
+	 * (last seq done << 1) | 1 (mapped host memory). */
 	const ResidentHostCmd* cmd;
 	ResidentCmd* bcast;
 	uint32_t* doneWords;

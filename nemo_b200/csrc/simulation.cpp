@@ -607,7 +607,7 @@ Simulation::construct(const Network& net, const Configuration& conf, const Shard
 	m_net.rngAhead = (uint4*) alloc(size_t(2) * m_nDev * 16);
 	m_net.fstim = (uint32_t*) alloc(size_t(m_net.nWords) * 4);
 	m_net.stats = (unsigned long long*) alloc(4 * 8);
-	m_net.barrier = (unsigned*) alloc(4 * 4);
+	m_net.barrier = (unsigned*) alloc(8 * 4);
 	m_net.firedList = (uint32_t*) alloc(size_t(2) * B * ownN * 4);
 	m_net.firedCnt = (uint32_t*) alloc(size_t(2) * B * 4);
 	m_net.postList = (uint2*) alloc(size_t(2) * B * postStride * 8);
@@ -1128,7 +1128,8 @@ Simulation::launchResident(uint32_t seq)
 	launchCycles(a, m_stream);
 	NEMO_CUDA(cudaGetLastError());
 	m_inline.nf = m_inline.ni = 0;
-	m_pendingGather = true;
+	/* the launch gathers every cycle it updates */
+	m_pendingGather = false;
 	m_resident = true;
 }
 
@@ -1213,7 +1214,7 @@ Simulation::stepResident(const unsigned* fstim, size_t nf, const unsigned* inidx
 }
 
 /* End the resident launch, if any: an exit command, then the stream drains.
- * The last cycle's gathering stays pending. */
+ * Its last cycle is gathered. */
 void
 Simulation::stopResident()
 {

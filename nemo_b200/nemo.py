@@ -118,6 +118,10 @@ class Library:
             fn = getattr(self.dll, name)
             fn.restype = restype
             fn.argtypes = argtypes
+        # nemo_step with its arrays as bytes objects (Simulation.step)
+        self.step_bytes = self.dll["nemo_step"]
+        self.step_bytes.restype = c_int
+        self.step_bytes.argtypes = [c_void_p, c_char_p, c_size_t, c_char_p, c_char_p, c_size_t, c_void_p, c_void_p]
         cls._cache[path] = self
         return self
 
@@ -322,22 +326,23 @@ class Simulation:
     def step(self, fstim=(), istim=()):
         """One 1 ms cycle. fstim: neuron indices forced to fire; istim: sequence
         of (neuron, current) pairs. Returns the fired neurons (uint32 array)."""
-        f = _u32(fstim) if len(fstim) else None
+        # a closed loop makes this call every cycle: arguments as bytes objects
+        # (their buffers are passed) and the fired list as one copy, about 5 us
+        # a call less than array and pointer objects
+        f = np.asarray(fstim, dtype=np.uint32).tobytes() if len(fstim) else None
         if len(istim):
-            inidx = _u32([p[0] for p in istim])
-            icur = _f32([p[1] for p in istim])
+            inidx = np.asarray([p[0] for p in istim], dtype=np.uint32).tobytes()
+            icur = np.asarray([p[1] for p in istim], dtype=np.float32).tobytes()
         else:
             inidx = icur = None
-        self.lib.call("nemo_step", self.handle,
-                      _ptr(f, c_uint) if f is not None else None, 0 if f is None else f.size,
-                      _ptr(inidx, c_uint) if inidx is not None else None,
-                      _ptr(icur, c_float) if icur is not None else None,
-                      0 if inidx is None else inidx.size,
-                      byref(self._fired), byref(self._nfired))
+        status = self.lib.step_bytes(self.handle, f, len(f) // 4 if f else 0, inidx, icur,
+                                     len(inidx) // 4 if inidx else 0, byref(self._fired), byref(self._nfired))
+        if status != NEMO_OK:
+            raise NemoError(status, self.lib.dll.nemo_strerror().decode(errors="replace"))
         n = self._nfired.value
         if n == 0:
             return np.zeros(0, dtype=np.uint32)
-        return np.ctypeslib.as_array(self._fired, shape=(n,)).copy()
+        return np.frombuffer(bytearray(ctypes.string_at(self._fired, 4 * n)), dtype=np.uint32)
 
     def apply_stdp(self, reward):
         self.lib.call("nemo_apply_stdp", self.handle, float(reward))
