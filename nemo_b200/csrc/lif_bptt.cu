@@ -871,6 +871,10 @@ k_adjoint(const __grid_constant__ Net n, const __grid_constant__ Adjoint a)
 						turn(e, ring[pos & uint32_t(RING - 1)], ring[(pos + 1u) & uint32_t(RING - 1)]);
 						__syncwarp(live);
 					}
+					/* the copies asked for past the run's end: the next step
+					 * writes the same places, and copies have no order of their
+					 * own */
+					asm volatile("cp.async.wait_all;" ::: "memory");
 				}
 			}
 		}
