@@ -266,6 +266,9 @@ k_dw_relaxed(Net n, int segStart, int segEnd, const float* guSeg, const float* s
 
 const int PART_STEPS = 64;
 const int PART_WARPS = 8;
+/* shared memory of a block at PART_STEPS steps (a step's row and a cell a
+ * lane), the most a call uses */
+const size_t PART_SMEM = size_t(PART_WARPS) * (PART_STEPS * 32 + 32) * 4;
 
 /* parts of a segment of `steps` steps and the steps of each (the last one
  * may have fewer) */
@@ -1163,6 +1166,25 @@ adjointKernel(int tw)
 	return tw == 8 ? (const void*) k_adjoint<8> : (tw == 16 ? (const void*) k_adjoint<16> : (const void*) k_adjoint<32>);
 }
 
+/* A kernel may use that much dynamic shared memory on the current device:
+ * the attribute is the device's, shared by all threads, so it is set once, to
+ * the most any call needs, and stays. False: a device with less. */
+static bool
+allowShared(const void* kernel, size_t smem)
+{
+	static std::mutex lock;
+	static std::map<std::pair<int, const void*>, bool> known;
+	int dev = 0;
+	NEMO_CUDA(cudaGetDevice(&dev));
+	std::lock_guard<std::mutex> guard(lock);
+	const std::pair<int, const void*> key(dev, kernel);
+	auto it = known.find(key);
+	if(it != known.end()) return it->second;
+	const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+	if(e != cudaSuccess) (void) cudaGetLastError();
+	return known[key] = e == cudaSuccess;
+}
+
 /* blocks of a kernel with that much shared memory that can run at once (one
  * an SM; 0: it does not fit), by device and kernel */
 static int
@@ -1179,11 +1201,9 @@ residentBlocks(const void* kernel, int threads, size_t smem)
 	int perSm = 0, sms = 0, coop = 0;
 	NEMO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
 	NEMO_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-	if(coop && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
-		(void) cudaGetLastError();   /* a device with less shared memory */
-		coop = 0;
+	if(coop && allowShared(kernel, smem)) {
+		NEMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, threads, smem));
 	}
-	if(coop) NEMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, threads, smem));
 	known[key] = perSm > 0 ? sms : 0;
 	return known[key];
 }
@@ -1466,8 +1486,8 @@ nemo_b200_lif_backward(const nemo_b200_lif_net* net, const float* w, const uint3
 		const unsigned gp = unsigned((n.N + lif::PART_WARPS - 1) / lif::PART_WARPS);
 		const size_t smemP = size_t(lif::PART_WARPS) * (size_t(L) * 32 + 32) * 4;
 		if(!relaxed) {
-			NEMO_CUDA(cudaFuncSetAttribute(lif::k_recompute, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemP)));
-			NEMO_CUDA(cudaFuncSetAttribute(lif::k_dw_events, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemP)));
+			lif::allowShared((const void*) lif::k_recompute, lif::PART_SMEM);
+			lif::allowShared((const void*) lif::k_dw_events, lif::PART_SMEM);
 		}
 		for(int sgi = segments - 1; sgi >= 0; --sgi) {
 			const int c0 = sgi * n.K, c1 = int(std::min<long>(n.T, long(c0) + n.K));

@@ -1,6 +1,9 @@
 """The differentiable form where its one-launch kernels step aside or take
-turns: under CUDA graph capture (its steps are then separate launches) and on
-two streams at once (its cooperative grids run one after another)."""
+turns: under CUDA graph capture (its steps are then separate launches), on two
+streams at once (its cooperative grids run one after another), and from two
+threads whose calls need different amounts of shared memory."""
+
+import threading
 
 import numpy as np
 import pytest
@@ -61,3 +64,38 @@ def test_two_streams():
     for i in range(2):
         for g in got[i]:
             _same(g, want[i])
+
+
+def test_two_threads_with_different_checkpoints():
+    # a network whose backward steps launch by launch and takes no turn; the
+    # segments' kernels use shared memory by the checkpoint interval (64 steps:
+    # 66 KB; 2 steps: 3 KB)
+    n, steps, trials = 40000, 64, 32
+    rng = np.random.default_rng(3)
+    tgt, pre = rng.integers(0, n, 3 * n), np.concatenate([rng.integers(0, n, 2 * n), n + rng.integers(0, 50, n)])
+    bits, _ = poisson_bits(steps, 50, trials, rate_hz=100.0, seed=3)
+    errors, grads = [], {}
+
+    def work(checkpoint, calls):
+        try:
+            net = LIFNetwork(n, 50, tgt, pre, checkpoint=checkpoint, bin_steps=8)
+            w = net.initial_weights(seed=3, scale_in=1.0)
+            with torch.cuda.stream(torch.cuda.Stream()):
+                d = torch.full((trials, steps // 8), 0.5, device="cuda")
+                _, saved = lif_forward(net, w, bits, trials)
+                for _ in range(calls):
+                    g = lif_backward(net, w, bits, trials, saved, d)
+                torch.cuda.current_stream().synchronize()
+            grads[checkpoint] = g
+        except Exception as e:   # reported by the main thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=a) for a in ((64, 30), (2, 60))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    # the same terms, grouped by segment
+    assert grads[2].norm() > 0
+    assert (grads[64].double() - grads[2].double()).norm() <= REL * grads[2].double().norm()
