@@ -249,7 +249,14 @@ nemo_status_t nemo_b200_host_bytes(nemo_simulation_t sim, unsigned long long out
  * (rowptr/pre: pre < N a recurrent neuron, whose spike arrives one step
  * later; pre >= N input channel pre - N, same step), and the recurrent ones
  * also by source (colptr/post/wpos, wpos the index in pre/w). Return a status;
- * nemo_b200_lif_error describes a failure. No counterpart in the reference. */
+ * nemo_b200_lif_error describes a failure. No counterpart in the reference.
+ *
+ * On a stream that is not being captured the calls launch kernels whose blocks
+ * wait for one another. Such kernels and those of the simulations (several
+ * cycles a launch, or nemo_step's resident launch) run one after another on a
+ * device, from whatever threads and streams: the stream of a call waits for the
+ * launches before it, and a resident launch of nemo_step is ended first; its
+ * simulation steps launch by launch while the others are in flight. */
 typedef struct nemo_b200_lif_net {
 	int N;          /* neurons */
 	int C;          /* input channels */

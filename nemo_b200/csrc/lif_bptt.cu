@@ -45,6 +45,7 @@
 #include <nemo_b200.h>
 
 #include "common.hpp"
+#include "device_turn.hpp"
 
 namespace nemo_b200 {
 namespace lif {
@@ -1277,7 +1278,7 @@ planForward(const Net& n)
 
 /* A stream that is being captured (or cannot tell) takes the launches whose
  * blocks never wait for one another: two graphs may run at once, and nothing
- * then orders their launches (Turn). */
+ * then orders their launches (DeviceTurn). */
 static bool
 capturing(cudaStream_t st)
 {
@@ -1289,35 +1290,13 @@ capturing(cudaStream_t st)
 	return status != cudaStreamCaptureStatusNone;
 }
 
-/* The kernels whose blocks wait for one another run one after another on a
- * device, whatever their streams: a call's launches wait for the last such
- * call's (two grids that each hold some of the SMs could otherwise each wait
- * for blocks of their own that cannot start). Held from before the first
- * launch to after the last. */
-class Turn {
-public:
-	explicit Turn(cudaStream_t st) : m_stream(st), m_guard(s_lock)
-	{
-		int dev = 0;
-		NEMO_CUDA(cudaGetDevice(&dev));
-		cudaEvent_t& e = s_event[dev];
-		if(e == nullptr) NEMO_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-		m_event = e;
-		NEMO_CUDA(cudaStreamWaitEvent(st, e, 0));
-	}
-	~Turn() { cudaEventRecord(m_event, m_stream); }
-	Turn(const Turn&) = delete;
-	Turn& operator=(const Turn&) = delete;
-
-private:
-	static std::mutex s_lock;
-	static std::map<int, cudaEvent_t> s_event;
-	cudaStream_t m_stream;
-	std::lock_guard<std::mutex> m_guard;
-	cudaEvent_t m_event;
-};
-std::mutex Turn::s_lock;
-std::map<int, cudaEvent_t> Turn::s_event;
+static int
+currentDevice()
+{
+	int dev = 0;
+	NEMO_CUDA(cudaGetDevice(&dev));
+	return dev;
+}
 
 static void
 validate(const Net& n)
@@ -1422,8 +1401,8 @@ nemo_b200_lif_forward(const nemo_b200_lif_net* net, const float* w, const uint32
 		if(plan.blocks) {
 			NEMO_CUDA(cudaMemsetAsync(k.barrier, 0, 8, st));
 			lif::Forward f = {w, in_bits, s_bits, v_ckpt, counts, plan.perBlock, plan.cached, k.barrier};
-			std::unique_ptr<lif::Turn> turn;
-			if(plan.blocks > 1) turn.reset(new lif::Turn(st));
+			std::unique_ptr<DeviceTurn> turn;
+			if(plan.blocks > 1) turn.reset(new DeviceTurn(lif::currentDevice(), st));
 			void* params[] = {&n, &f};
 			NEMO_CUDA(cudaLaunchCooperativeKernel(plan.kernel, dim3(unsigned(plan.blocks)),
 					dim3(unsigned(lif::FWD_THREADS)), params, lif::FWD_SMEM, st));
@@ -1457,7 +1436,7 @@ nemo_b200_lif_backward(const nemo_b200_lif_net* net, const float* w, const uint3
 		const int g = lif::grid(n.N);
 		const lif::AdjointPlan plan = relaxed || lif::capturing(st) ? lif::AdjointPlan() : lif::planAdjoint(n);
 		const int tw = plan.tw;
-		std::unique_ptr<lif::Turn> turn;
+		std::unique_ptr<DeviceTurn> turn;
 		NEMO_CUDA(cudaMemsetAsync(k.barrier, 0, 8, st));
 		lif::Adjoint adj = {};
 		if(plan.parts) {
@@ -1476,7 +1455,7 @@ nemo_b200_lif_backward(const nemo_b200_lif_net* net, const float* w, const uint3
 			adj.guSeg = k.guSeg;
 			adj.dcounts = dcounts;
 			adj.barrier = k.barrier;
-			turn.reset(new lif::Turn(st));
+			turn.reset(new DeviceTurn(lif::currentDevice(), st));
 		} else if(n.nnzRec) {
 			lif::k_gather_out<<<g, lif::THREADS, 0, st>>>(n, n.nnzRec, w, k.wOut);
 		}

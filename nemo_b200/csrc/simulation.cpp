@@ -753,12 +753,8 @@ Simulation::~Simulation()
 void
 Simulation::release()
 {
-	if(m_resident && m_rcmd) {
-		/* end the resident launch without raising (destructor) */
-		postCommand(++m_rseq, RESIDENT_EXIT);
-		m_resident = false;
-	}
-	releaseResidentDevice();
+	endStay();
+	DeviceTurn::leave(m_device, this);
 	if(m_stream) cudaStreamSynchronize(STREAM(m_stream));
 	destroyGraph();
 	for(void** ev : {&m_evOut, &m_evIn, &m_evStaged}) {
@@ -1050,49 +1046,13 @@ Simulation::mapInline(const unsigned* fstim, size_t nf, const unsigned* inidx, c
 	return true;
 }
 
-/* The simulation whose resident launch is on each device, if any. Two
- * resident launches must not share a device: each occupies an SM with every
- * block, and when both are partly resident, each one's blocks can wait for
- * its first block, which cannot start while the other's hold the SMs. */
-static std::mutex g_residentLock;
-static std::map<int, Simulation*> g_residentOwner;
-
-void
-Simulation::claimResidentDevice()
-{
-	Simulation* other = nullptr;
-	{
-		std::lock_guard<std::mutex> lock(g_residentLock);
-		auto it = g_residentOwner.find(m_device);
-		if(it != g_residentOwner.end() && it->second != this) other = it->second;
-		g_residentOwner[m_device] = this;
-	}
-	if(other) {
-		/* its error, if any, is its own: that simulation reports it on its
-		 * next call */
-		try {
-			other->stopResident();
-		} catch(...) {
-		}
-	}
-}
-
-void
-Simulation::releaseResidentDevice()
-{
-	std::lock_guard<std::mutex> lock(g_residentLock);
-	auto it = g_residentOwner.find(m_device);
-	if(it != g_residentOwner.end() && it->second == this) g_residentOwner.erase(it);
-}
-
 /* The resident step kernel's launch for command `seq`, whose stimulus is
  * m_inline; the pending gathering of the last cycle, if any, is its first
  * phase's. The launch keeps the current slots in shared memory while it
- * stays. */
+ * stays. With the device's turn and m_stayLock held. */
 void
 Simulation::launchResident(uint32_t seq)
 {
-	claimResidentDevice();
 	if(m_rcmd == nullptr) {
 		NEMO_CUDA(cudaHostAlloc((void**) &m_rcmd, sizeof(ResidentHostCmd), cudaHostAllocMapped));
 		NEMO_CUDA(cudaHostGetDevicePointer((void**) &m_dRcmd, m_rcmd, 0));
@@ -1157,42 +1117,26 @@ Simulation::postCommand(uint32_t seq, uint32_t op)
 	}
 }
 
-/* One cycle through the resident kernel; false when the stimulus does not
- * fit the command (nothing done: the caller takes the ordinary path). */
+/* Wait for the done word of command `seq` (m_stayLock held); false when the
+ * launch ended (idle) before the command. */
 bool
-Simulation::stepResident(const unsigned* fstim, size_t nf, const unsigned* inidx, const float* icur, size_t ni)
+Simulation::awaitCommand(uint32_t seq)
 {
-	if(!mapInline(fstim, nf, inidx, icur, ni)) return false;
-	if(!fitsCommand()) {
-		m_inline.nf = m_inline.ni = 0;
-		return false;
-	}
-	const uint32_t seq = ++m_rseq;
-	if(!m_resident) {
-		launchResident(seq);
-	} else {
-		postCommand(seq, RESIDENT_STEP);
-		m_inline.nf = m_inline.ni = 0;
-	}
 	volatile const uint32_t* done = m_rdone;
 	const auto start = std::chrono::steady_clock::now();
-	for(uint64_t spin = 0;; ++spin) {
-		if(done[0] == seq) break;
+	for(uint64_t spin = 0; done[0] != seq; ++spin) {
 		const uint32_t exitInfo = done[1];
 		if(exitInfo != 0u && (exitInfo >> 1) < seq) {
-			/* the launch ended (idle) before this command: run it in a new one */
 			NEMO_CUDA(cudaStreamSynchronize(STREAM(m_stream)));
 			m_resident = false;
 			if(m_stepWords[0] != 0) {
 				fail(NEMO_CUDA_ASSERTION_FAILURE, "step kernel: a grid barrier timed out; the simulation state is invalid");
 			}
-			mapInline(fstim, nf, inidx, icur, ni);
-			launchResident(seq);
-			continue;
+			return false;
 		}
 		if((spin & 4095u) == 4095u) {
 			const cudaError_t e = cudaStreamQuery(STREAM(m_stream));
-			if(e != cudaErrorNotReady) {
+			if(e != cudaErrorNotReady && done[0] != seq && done[1] == 0u) {
 				/* the launch is over without this command done: a fault or a
 				 * barrier timeout */
 				m_resident = false;
@@ -1205,6 +1149,54 @@ Simulation::stepResident(const unsigned* fstim, size_t nf, const unsigned* inidx
 		}
 	}
 	std::atomic_thread_fence(std::memory_order_acquire);
+	return true;
+}
+
+/* One cycle through the resident kernel; false when the stimulus does not
+ * fit the command, or when the device's turn is another caller's (nothing
+ * done: the caller takes the ordinary path). */
+bool
+Simulation::stepResident(const unsigned* fstim, size_t nf, const unsigned* inidx, const float* icur, size_t ni)
+{
+	if(!mapInline(fstim, nf, inidx, icur, ni)) return false;
+	if(!fitsCommand()) {
+		m_inline.nf = m_inline.ni = 0;
+		return false;
+	}
+	if(m_turnWanted == nullptr) m_turnWanted = DeviceTurn::wanted(m_device);
+	bool done = false;
+	if(m_resident && m_turnWanted->load() == 0) {
+		std::lock_guard<std::mutex> guard(m_stayLock);
+		if(m_resident) {
+			const uint32_t seq = ++m_rseq;
+			postCommand(seq, RESIDENT_STEP);
+			/* when the launch ended before the command: in a new one */
+			done = awaitCommand(seq);
+		}
+	}
+	if(!done) {
+		bool stayed = false;
+		if(!m_resident) {
+			raiseStayError();
+			uint32_t seq = 0;
+			stayed = DeviceTurn::tryStay(m_device, this, [&] {
+				std::lock_guard<std::mutex> guard(m_stayLock);
+				seq = ++m_rseq;
+				launchResident(seq);
+			});
+			if(stayed) {
+				std::lock_guard<std::mutex> guard(m_stayLock);
+				if(!awaitCommand(seq)) {
+					fail(NEMO_CUDA_ASSERTION_FAILURE, "resident step kernel ended without completing the cycle");
+				}
+			}
+		}
+		if(!stayed) {
+			m_inline.nf = m_inline.ni = 0;
+			return false;
+		}
+	}
+	m_inline.nf = m_inline.ni = 0;
 	m_cycle++;
 	m_stateDirty = true;
 	decodeStepList(m_fired);
@@ -1213,19 +1205,51 @@ Simulation::stepResident(const unsigned* fstim, size_t nf, const unsigned* inidx
 	return true;
 }
 
-/* End the resident launch, if any: an exit command, then the stream drains.
- * Its last cycle is gathered. */
+/* End the resident launch (m_stayLock held): an exit command, then the stream
+ * drains. Its last cycle is gathered. */
 void
-Simulation::stopResident()
+Simulation::endLaunch()
 {
-	if(!m_resident) return;
 	postCommand(++m_rseq, RESIDENT_EXIT);
 	m_resident = false;
-	releaseResidentDevice();
 	NEMO_CUDA(cudaStreamSynchronize(STREAM(m_stream)));
 	NEMO_CUDA(cudaGetLastError());
 	if(m_stepWords[0] != 0) {
 		fail(NEMO_CUDA_ASSERTION_FAILURE, "step kernel: a grid barrier timed out; the simulation state is invalid");
+	}
+}
+
+/* The error of a stay that another thread ended */
+void
+Simulation::raiseStayError()
+{
+	std::unique_lock<std::mutex> guard(m_stayLock);
+	if(m_stayError) {
+		std::exception_ptr e = m_stayError;
+		m_stayError = nullptr;
+		guard.unlock();
+		std::rethrow_exception(e);
+	}
+}
+
+void
+Simulation::stopResident()
+{
+	{
+		std::lock_guard<std::mutex> guard(m_stayLock);
+		if(m_resident) endLaunch();
+	}
+	raiseStayError();
+}
+
+void
+Simulation::endStay() noexcept
+{
+	std::lock_guard<std::mutex> guard(m_stayLock);
+	try {
+		if(m_resident) endLaunch();
+	} catch(...) {
+		m_stayError = std::current_exception();
 	}
 }
 
@@ -1554,6 +1578,7 @@ Simulation::run(unsigned cycles, uint32_t* firedCounts, uint64_t* events)
 		}
 		flushPending();
 	} else {
+		DeviceTurn turn(m_device, stream, this);
 		launchBlock(m_cycle, cycles);
 		m_cycle += cycles;
 	}
@@ -1655,16 +1680,19 @@ Simulation::runGraph(unsigned cycles, unsigned cyclesPerLaunch, int* usedGraph)
 	}
 	uint64_t counter = m_cycle;
 	NEMO_CUDA(cudaMemcpyAsync(m_dCycleCounter, &counter, 8, cudaMemcpyHostToDevice, stream));
-	if(m_graphUsable && m_graphExec) {
-		NEMO_CUDA(cudaGraphLaunch(static_cast<cudaGraphExec_t>(m_graphExec), stream));
-		if(usedGraph) *usedGraph = 1;
-	} else {
-		for(unsigned done = 0; done < cycles; done += cyclesPerLaunch) {
-			a.cycles = std::min(cyclesPerLaunch, cycles - done);
-			launchCycles(a, m_stream);
-			NEMO_CUDA(cudaGetLastError());
+	{
+		DeviceTurn turn(m_device, stream, this);
+		if(m_graphUsable && m_graphExec) {
+			NEMO_CUDA(cudaGraphLaunch(static_cast<cudaGraphExec_t>(m_graphExec), stream));
+			if(usedGraph) *usedGraph = 1;
+		} else {
+			for(unsigned done = 0; done < cycles; done += cyclesPerLaunch) {
+				a.cycles = std::min(cyclesPerLaunch, cycles - done);
+				launchCycles(a, m_stream);
+				NEMO_CUDA(cudaGetLastError());
+			}
+			if(usedGraph) *usedGraph = 0;
 		}
-		if(usedGraph) *usedGraph = 0;
 	}
 	m_cycle += cycles;
 	m_stateDirty = true;
@@ -1700,6 +1728,8 @@ Simulation::autotuneShape(unsigned trialCycles, double ms[6])
 	NEMO_CUDA(cudaEventCreate(&e0));
 	NEMO_CUDA(cudaEventCreate(&e1));
 	for(int k = 0; k < 6; ++k) ms[k] = k < 3 * nRuns ? 1e300 : 0.0;
+	/* every trial with the device's other waiting grids behind it */
+	std::unique_ptr<DeviceTurn> turn(new DeviceTurn(m_device, stream, this));
 	for(int round = 0; round < 2; ++round) {
 		for(int r = 0; r < nRuns; ++r) {
 			for(int k = 0; k < 3; ++k) {
@@ -1718,6 +1748,7 @@ Simulation::autotuneShape(unsigned trialCycles, double ms[6])
 			}
 		}
 	}
+	turn.reset();
 	for(int r = 0; r < nRuns; ++r) {
 		for(int k = 0; k < 3; ++k) {
 			if(ms[3 * r + k] < bestMs) {
@@ -2074,15 +2105,18 @@ Simulation::timedSteps(unsigned steps, unsigned cyclesPerStep, bool apply, float
 	cudaEvent_t e0, e1;
 	NEMO_CUDA(cudaEventCreate(&e0));
 	NEMO_CUDA(cudaEventCreate(&e1));
-	NEMO_CUDA(cudaEventRecord(e0, stream));
-	for(unsigned s = 0; s < steps; ++s) {
-		launchBlock(m_cycle, cyclesPerStep);
-		m_cycle += cyclesPerStep;
-		if(apply && m_nrcm) {
-			launchApply(fx);
+	{
+		DeviceTurn turn(m_device, stream, this);
+		NEMO_CUDA(cudaEventRecord(e0, stream));
+		for(unsigned s = 0; s < steps; ++s) {
+			launchBlock(m_cycle, cyclesPerStep);
+			m_cycle += cyclesPerStep;
+			if(apply && m_nrcm) {
+				launchApply(fx);
+			}
 		}
+		NEMO_CUDA(cudaEventRecord(e1, stream));
 	}
-	NEMO_CUDA(cudaEventRecord(e1, stream));
 	NEMO_CUDA(cudaEventSynchronize(e1));
 	float ms = 0;
 	NEMO_CUDA(cudaEventElapsedTime(&ms, e0, e1));
@@ -2113,10 +2147,13 @@ Simulation::profile(unsigned cycles, float reward, double out[10])
 	NEMO_CUDA(cudaEventCreate(&e2));
 	uint64_t before[4], after[4];
 	readStats(before);
-	NEMO_CUDA(cudaEventRecord(e0, stream));
-	launchBlock(m_cycle, cycles);
-	m_cycle += cycles;
-	NEMO_CUDA(cudaEventRecord(e1, stream));
+	{
+		DeviceTurn turn(m_device, stream, this);
+		NEMO_CUDA(cudaEventRecord(e0, stream));
+		launchBlock(m_cycle, cycles);
+		m_cycle += cycles;
+		NEMO_CUDA(cudaEventRecord(e1, stream));
+	}
 	if(m_stdpOn && m_nrcm) {
 		launchApply(toFix(reward, m_fbits));
 		m_fcmHostValid = false;
@@ -2165,8 +2202,11 @@ Simulation::trace(unsigned cycles, double out[24])
 	a.cycles = cycles;
 	a.trace = dTrace;
 	for(int gi = 0; gi < a.ngroups; ++gi) a.groups[gi].timerBase = uint32_t(m_timerBase);
-	launchCycles(a, m_stream);
-	NEMO_CUDA(cudaGetLastError());
+	{
+		DeviceTurn turn(m_device, stream, this);
+		launchCycles(a, m_stream);
+		NEMO_CUDA(cudaGetLastError());
+	}
 	m_cycle += cycles;
 	m_stateDirty = true;
 	std::vector<unsigned long long> h(words);

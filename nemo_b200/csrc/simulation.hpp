@@ -6,11 +6,15 @@
  * 45-147, cpu/Simulation.cpp, cuda/Simulation.cpp), with the per-cycle work
  * done by the persistent kernel of kernels.cu. */
 
+#include <atomic>
 #include <chrono>
 #include <cstdint>
+#include <exception>
+#include <mutex>
 #include <unordered_map>
 #include <vector>
 
+#include "device_turn.hpp"
 #include "kernels.hpp"
 #include "network.hpp"
 #include "plugin.hpp"
@@ -45,14 +49,13 @@ Network shardNetwork(const Network& net, unsigned rank, unsigned world, ShardSpe
  * at most one, lower ranks take the extra ones. */
 void shardWarps(uint32_t totalWarps, unsigned rank, unsigned world, uint32_t* lo, uint32_t* hi);
 
-class Simulation {
+class Simulation final : private Stay {
 public:
 	Simulation(const Network& net, const Configuration& conf, const ShardSpec* shard = nullptr);
 	~Simulation();
 
 	/* End this simulation's resident step launch, if any (every call but
-	 * step() does it first; a resident launch of another simulation on the
-	 * same device does it too) */
+	 * step() does it first; another caller's turn on the device does it too) */
 	void stopResident();
 
 	/* One cycle with stimulus; returns the fired neurons (user indices) in
@@ -365,15 +368,23 @@ private:
 	bool mapInline(const unsigned* fstim, size_t nf, const unsigned* inidx, const float* icur, size_t ni);
 	bool fitsCommand() const { return 3u + m_inline.nf + 2u * m_inline.ni <= 3u * RESIDENT_CHUNKS; }
 	void launchResident(uint32_t seq);
-	void claimResidentDevice();
-	void releaseResidentDevice();
-	bool m_resident = false;            /* a resident launch is on the stream */
+	bool awaitCommand(uint32_t seq);
+	void endLaunch();
+	void endStay() noexcept override;
+	void raiseStayError();
+	/* the resident launch's command buffer and the members below, between this
+	 * simulation's thread and another one that ends the stay (endStay). Only
+	 * this simulation's thread makes m_resident true. */
+	std::mutex m_stayLock;
+	std::atomic<bool> m_resident{false};   /* a resident launch is on the stream */
+	std::exception_ptr m_stayError;     /* of a stay that another thread ended: raised by the next call */
+	const std::atomic<int>* m_turnWanted = nullptr;   /* DeviceTurn::wanted */
 	bool m_residentOn = true;           /* nemo_step may use resident stepping */
 	uint32_t m_rseq = 0;                /* the last command number */
 	/* bytes of the per-cycle steps' inputs and outputs across the bus:
 	 * stimulus (resident command chunks, or the staged copies and kernel
 	 * parameters) and the step lists read back (hostBytes) */
-	uint64_t m_bytesIn = 0;
+	std::atomic<uint64_t> m_bytesIn{0};
 	uint64_t m_bytesOut = 0;
 	ResidentHostCmd* m_rcmd = nullptr;  /* mapped host memory */
 	ResidentHostCmd* m_dRcmd = nullptr; /* its device address */
