@@ -51,10 +51,12 @@ def _headers_mtime():
 def _compile(src, verbose=False):
     path = os.path.join(CSRC, src)
     obj = os.path.join(BUILD, src + ".o")
-    if os.path.exists(obj) and os.path.getmtime(obj) >= max(os.path.getmtime(path), _headers_mtime()):
+    report = obj + ".ptxas"   # kernels: registers and spills by function
+    if os.path.exists(obj) and os.path.getmtime(obj) >= max(os.path.getmtime(path), _headers_mtime()) \
+            and (os.path.exists(report) or not src.endswith(".cu")):
         return obj
     if src.endswith(".cu"):
-        cmd = [NVCC] + NVCC_FLAGS + ["-c", path, "-o", obj]
+        cmd = [NVCC] + NVCC_FLAGS + ["-Xptxas", "-v", "-c", path, "-o", obj]
     else:
         cmd = [CXX] + CXX_FLAGS + ["-c", path, "-o", obj]
     if verbose:
@@ -62,6 +64,9 @@ def _compile(src, verbose=False):
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("compiling %s failed:\n%s%s" % (src, r.stdout, r.stderr))
+    if src.endswith(".cu"):
+        with open(report, "w") as f:
+            f.write(r.stderr)
     return obj
 
 

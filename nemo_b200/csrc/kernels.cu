@@ -572,9 +572,9 @@ __device__ __forceinline__ bool modelHH(const NetDev& net, const GroupDev& g, ui
 	return fired;
 }
 
-/* modelHH with registers of its own: the step kernel with the step-list and
- * resident code has none to spare, and spilled the substep's
- * (555 us a cycle of the mixed network against 495) */
+/* modelHH with registers of its own: where a step list is written the kernel
+ * has none to spare for the substep (the mixed network of 50,000 neurons, 20
+ * cycles through nemo_step: 11.39 ms against 11.70 with the model in place) */
 __device__ __noinline__ bool callHH(const NetDev& net, const GroupDev& g, uint32_t i, float E, float I, uint32_t stimWord,
 		uint32_t cycle, uint32_t lane)
 {
@@ -926,17 +926,26 @@ __device__ __forceinline__ void writeStepList(const NetDev& net, uint32_t* hostW
 	if(threadIdx.x == 0) hostWords[1] = done;
 }
 
-/* k_cycles: see kernels.hpp for the phase structure. HOST: the launch may
- * write a step list to host memory or stay resident (CycleArgs::hostWords,
- * cmd); launches that do neither use the instantiation without that code,
- * which leaves the rest more registers. HH: the network has Hodgkin-Huxley
- * neurons; the others run without that model's code for the same reason. The forward regions and
+/* What a launch of the step kernel does beyond its cycles: nothing (several
+ * cycles, or a pending gathering; the only one that can be traced), write one
+ * cycle's step list to host memory (CycleArgs::hostWords), or stay and take
+ * its cycles from commands (CycleArgs::cmd) */
+enum { MODE_RUN, MODE_STEP, MODE_RESIDENT };
+
+/* k_cycles: see kernels.hpp for the phase structure. The 64 registers of
+ * 1024 threads are just enough for one of the modes, so each has an
+ * instantiation of its own; one for both kinds of steps, with the trace's
+ * code, spilled (184 bytes of loads a thread against 0, and 28 for a single
+ * step): a call of nemo_step in a loop took 31.6 us on 100k neurons with STDP
+ * and 14.2 on 1,000 without, now 28.7 and 13.5. HH: the network has
+ * Hodgkin-Huxley neurons; the others run without that model's code for the
+ * same reason. The forward regions and
  * the reverse-matrix arrays are streamed with evict-first loads and stores
  * (__ldcs / __stcs), so that they do not push the randomly read firing
  * history, segment offsets and noise tables out of L2. SMEM: the owned current
  * slots live in dynamic shared memory as int32 E/I pairs,
  * sAcc[slot * ownN + local]; otherwise every access goes to net.acc. */
-template<bool SMEM, unsigned T, bool HOST, bool HH>
+template<bool SMEM, unsigned T, int MODE, bool HH>
 __global__ void __launch_bounds__(T, 1)
 k_cycles(const __grid_constant__ CycleArgs A)
 {
@@ -947,6 +956,8 @@ k_cycles(const __grid_constant__ CycleArgs A)
 	__shared__ uint32_t sNFired, sNPost, sWork, sLast;
 	__shared__ unsigned long long sEvents, sPushed, sVisits;
 
+	const bool HOST = MODE != MODE_RUN;           /* writes step lists */
+	const bool resident = MODE == MODE_RESIDENT;
 	const NetDev& net = A.net;
 	const uint32_t tid = threadIdx.x;
 	const uint32_t lane = tid & 31u;
@@ -1005,12 +1016,11 @@ k_cycles(const __grid_constant__ CycleArgs A)
 	/* resident stepping (CycleArgs::cmd): an update phase and its gather phase
 	 * per command until an exit command or the idle limit; nothing stays
 	 * pending but the delay-1 arrivals in the inbox */
-	const bool resident = HOST && A.cmd != nullptr;
 	const bool lastPending = resident || (A.carry & 2u) != 0u;
 	const uint32_t phases = resident ? 0xffffffffu : A.cycles + (lastPending ? 0u : 1u);
 	/* a resident launch's count of block arrivals after the updates when it
 	 * started */
-	const unsigned doneBase = HOST ? *(volatile unsigned*) &net.barrier[5] : 0u;
+	const unsigned doneBase = resident ? *(volatile unsigned*) &net.barrier[5] : 0u;
 	const uint32_t barriers = lastPending && A.cycles ? A.cycles - 1u : A.cycles;
 	uint32_t passed = 0;   /* grid barriers passed */
 	uint32_t k = 0;        /* the update (resident: the command), counted from the launch's start */
@@ -1069,7 +1079,7 @@ k_cycles(const __grid_constant__ CycleArgs A)
 			if(warp == 1 && net.stdp) warpPrefix(net.postCnt + par * B, B, sPreP, lane);
 		}
 		__syncthreads();
-		unsigned long long* trace = A.trace ? A.trace + (size_t(k) * B + b) * TRACE_WORDS : nullptr;
+		unsigned long long* trace = !HOST && A.trace ? A.trace + (size_t(k) * B + b) * TRACE_WORDS : nullptr;
 		if(trace && tid == 0) trace[0] = globalTimer();
 
 		/* ---- neuron update of cycle t for the owned neurons, by the first
@@ -1517,7 +1527,7 @@ k_cycles(const __grid_constant__ CycleArgs A)
 			if(sVisits) atomicAdd(&net.stats[1], sVisits);
 		}
 		if(trace && tid == 0) trace[3] = globalTimer();
-		if(HOST && A.hostWords && doUpdate) {
+		if(HOST && doUpdate) {
 			/* the step's list, by the block whose update arrives last: the
 			 * count starts again for the next step (which the host starts after
 			 * this one's list), or in a resident launch goes on */
@@ -1553,13 +1563,13 @@ k_cycles(const __grid_constant__ CycleArgs A)
 			if(b == 0) {
 				residentNext(A, seqK, k, warp, lane);
 			} else if(!residentWait(A, seqK, k)) {
-				if(HOST && A.hostWords && tid == 0) A.hostWords[0] = 1u;
+				if(HOST && tid == 0) A.hostWords[0] = 1u;
 				return;
 			}
 			if(*(volatile const uint32_t*) &A.bcast[(k + 1u) & 1u].op != RESIDENT_STEP) break;
 		} else if(!resident && k < barriers) {
 			if(!gridSync(net.barrier, barBase + (k + 1u) * B, A.timeoutNs)) {
-				if(HOST && A.hostWords && tid == 0) A.hostWords[0] = 1u;
+				if(HOST && tid == 0) A.hostWords[0] = 1u;
 				return;
 			}
 			passed++;
@@ -2013,27 +2023,34 @@ launchStimulusScratch(const NetDev& net, const uint32_t* scratch, uint32_t nf, u
 	k_stimulus_scratch<<<blocks, 256, 0, S(stream)>>>(net, scratch, nf, ni);
 }
 
-template<bool SMEM, bool HOST, bool HH>
+template<bool SMEM, int MODE, bool HH>
 static const void*
 cyclesKernelT(uint32_t threads)
 {
 	switch(threads) {
-		case 256: return (const void*) k_cycles<SMEM, 256, HOST, HH>;
-		case 512: return (const void*) k_cycles<SMEM, 512, HOST, HH>;
-		default: return (const void*) k_cycles<SMEM, 1024, HOST, HH>;
+		case 256: return (const void*) k_cycles<SMEM, 256, MODE, HH>;
+		case 512: return (const void*) k_cycles<SMEM, 512, MODE, HH>;
+		default: return (const void*) k_cycles<SMEM, 1024, MODE, HH>;
+	}
+}
+
+template<bool SMEM, bool HH>
+static const void*
+cyclesKernelM(uint32_t threads, int mode)
+{
+	switch(mode) {
+		case MODE_RUN: return cyclesKernelT<SMEM, MODE_RUN, HH>(threads);
+		case MODE_STEP: return cyclesKernelT<SMEM, MODE_STEP, HH>(threads);
+		default: return cyclesKernelT<SMEM, MODE_RESIDENT, HH>(threads);
 	}
 }
 
 /* the instantiation of the step kernel */
 static const void*
-cyclesKernel(bool smem, uint32_t threads, bool host, bool hh)
+cyclesKernel(bool smem, uint32_t threads, int mode, bool hh)
 {
-	if(smem) {
-		return host ? (hh ? cyclesKernelT<true, true, true>(threads) : cyclesKernelT<true, true, false>(threads))
-			: (hh ? cyclesKernelT<true, false, true>(threads) : cyclesKernelT<true, false, false>(threads));
-	}
-	return host ? (hh ? cyclesKernelT<false, true, true>(threads) : cyclesKernelT<false, true, false>(threads))
-		: (hh ? cyclesKernelT<false, false, true>(threads) : cyclesKernelT<false, false, false>(threads));
+	if(smem) return hh ? cyclesKernelM<true, true>(threads, mode) : cyclesKernelM<true, false>(threads, mode);
+	return hh ? cyclesKernelM<false, true>(threads, mode) : cyclesKernelM<false, false>(threads, mode);
 }
 
 /* The step kernel's plan: one 1024-thread block per SM (its registers allow
@@ -2066,16 +2083,19 @@ cyclesPlan(const std::vector<uint32_t>& warpCost, uint32_t slots, bool acc32, bo
 	const bool smem = acc32 && bytes <= SMEM_ACC_LIMIT;
 	/* the attribute is per device and shared by all simulations: set it to
 	 * the largest size any of them uses */
-	int perSm = 0, perSmHost = 0;
-	for(int v = 0; smem && v < 12; ++v) {
-		const uint32_t threads = v % 3 == 0 ? 1024u : (v % 3 == 1 ? 512u : 256u);
-		cudaFuncSetAttribute(cyclesKernel(true, threads, v / 3 % 2, v / 6), cudaFuncAttributeMaxDynamicSharedMemorySize,
-				int(SMEM_ACC_LIMIT));
-	}
+	int perSm = 1;
 	const size_t dyn = smem ? size_t(bytes) : 0;
-	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, cyclesKernel(smem, 1024, false, hh), 1024, dyn);
-	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSmHost, cyclesKernel(smem, 1024, true, hh), 1024, dyn);
-	perSm = std::min(perSm, perSmHost);
+	for(int mode : {MODE_RUN, MODE_STEP, MODE_RESIDENT}) {
+		for(uint32_t threads : {1024u, 512u, 256u}) {
+			if(smem) {
+				cudaFuncSetAttribute(cyclesKernel(true, threads, mode, hh), cudaFuncAttributeMaxDynamicSharedMemorySize,
+						int(SMEM_ACC_LIMIT));
+			}
+		}
+		int fit = 0;
+		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, cyclesKernel(smem, 1024, mode, hh), 1024, dyn);
+		perSm = std::min(perSm, fit);
+	}
 	*blocks = perSm >= 1 ? B : 0u;
 	*ownWarps = most;
 	*smemAcc = smem;
@@ -2089,7 +2109,8 @@ launchCycles(const CycleArgs& args, void* stream)
 	const bool smem = net.smemAcc && !args.globalAcc;
 	bool hh = false;
 	for(int g = 0; g < args.ngroups; ++g) hh = hh || args.groups[g].kind == 3;   /* MODEL_HH */
-	const void* kernel = cyclesKernel(smem, net.threads, args.hostWords || args.cmd, hh);
+	const int mode = args.cmd ? MODE_RESIDENT : (args.hostWords ? MODE_STEP : MODE_RUN);
+	const void* kernel = cyclesKernel(smem, net.threads, mode, hh);
 	const size_t bytes = smem ? size_t(net.slots) * net.ownWarps * 32u * 8u : 0;
 	const uint32_t threads = net.threads == 256u || net.threads == 512u ? net.threads : 1024u;
 	if(args.cycles <= 1u && (args.carry & 2u) && args.cmd == nullptr) {
