@@ -327,8 +327,8 @@ class Simulation:
         """One 1 ms cycle. fstim: neuron indices forced to fire; istim: sequence
         of (neuron, current) pairs. Returns the fired neurons (uint32 array)."""
         # a closed loop makes this call every cycle: arguments as bytes objects
-        # (their buffers are passed) and the fired list as one copy, about 5 us
-        # a call less than array and pointer objects
+        # (their buffers are passed) and the fired list copied as bytes, about 5
+        # us a call less than array and pointer objects
         f = np.asarray(fstim, dtype=np.uint32).tobytes() if len(fstim) else None
         if len(istim):
             inidx = np.asarray([p[0] for p in istim], dtype=np.uint32).tobytes()
@@ -342,7 +342,7 @@ class Simulation:
         n = self._nfired.value
         if n == 0:
             return np.zeros(0, dtype=np.uint32)
-        return np.frombuffer(bytearray(ctypes.string_at(self._fired, 4 * n)), dtype=np.uint32)
+        return np.frombuffer(ctypes.string_at(self._fired, 4 * n), dtype=np.uint32).copy()
 
     def apply_stdp(self, reward):
         self.lib.call("nemo_apply_stdp", self.handle, float(reward))

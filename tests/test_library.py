@@ -180,3 +180,20 @@ def test_cpp_api_simulation(tmp_path):
     r = subprocess.run([exe, "simulate"], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
     assert "ok ring" in r.stdout
+
+
+def test_step_returns_an_array_of_its_own(oracle_lib):
+    from nemo_b200.nemo import Configuration, Simulation
+    net = Network(oracle_lib)
+    net.add_neuron(net.add_neuron_type("Input"), np.arange(8, dtype=np.uint32))
+    conf = Configuration(oracle_lib)
+    conf.set_cpu_backend()
+    sim = Simulation(net, conf)
+    for f in ([], [3], [1, 2, 6]):
+        fired = sim.step(f)
+        assert fired.dtype == np.uint32 and fired.tolist() == f
+        # the caller's to change, in place and in size, and kept by later steps
+        assert fired.flags.owndata and fired.flags.writeable
+        fired.resize(len(f) + 2, refcheck=False)
+        sim.step([7])
+        assert fired[:len(f)].tolist() == f
