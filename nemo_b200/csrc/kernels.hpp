@@ -236,6 +236,12 @@ struct StdpRule {
 const uint32_t RESIDENT_STEP = 1;
 const uint32_t RESIDENT_EXIT = 2;
 const uint32_t RESIDENT_CHUNKS = 32;
+/* the largest command number: twice as many phases and the exit word (number
+ * << 1 | 1) stay within 32 bits. Past half of it a launch starts at 1 again */
+#ifndef NEMO_B200_RESIDENT_LAST
+#define NEMO_B200_RESIDENT_LAST 0x7ffffffeu
+#endif
+const uint32_t RESIDENT_LAST = NEMO_B200_RESIDENT_LAST;
 struct ResidentChunk {
 	uint32_t seq;
 	uint32_t w[3];

@@ -1046,12 +1046,12 @@ Simulation::mapInline(const unsigned* fstim, size_t nf, const unsigned* inidx, c
 	return true;
 }
 
-/* The resident step kernel's launch for command `seq`, whose stimulus is
- * m_inline; the pending gathering of the last cycle, if any, is its first
+/* The resident step kernel's launch for the next command (returns its number),
+ * whose stimulus is m_inline; the pending gathering of the last cycle, if any, is its first
  * phase's. The launch keeps the current slots in shared memory while it
  * stays. With the device's turn and m_stayLock held. */
-void
-Simulation::launchResident(uint32_t seq)
+uint32_t
+Simulation::launchResident()
 {
 	if(m_rcmd == nullptr) {
 		NEMO_CUDA(cudaHostAlloc((void**) &m_rcmd, sizeof(ResidentHostCmd), cudaHostAllocMapped));
@@ -1062,6 +1062,14 @@ Simulation::launchResident(uint32_t seq)
 		m_rbcast = (ResidentCmd*) alloc(2 * sizeof(ResidentCmd));
 		std::memset(m_rcmd, 0, sizeof(ResidentHostCmd));
 	}
+	if(m_rseq >= RESIDENT_LAST / 2) {
+		/* no launch reads either copy now: numbers of long ago must not be
+		 * taken for new ones */
+		std::memset(m_rcmd, 0, sizeof(ResidentHostCmd));
+		NEMO_CUDA(cudaMemsetAsync(m_rbcast, 0, 2 * sizeof(ResidentCmd), STREAM(m_stream)));
+		m_rseq = 0;
+	}
+	const uint32_t seq = ++m_rseq;
 	/* no command of this launch has run yet: done word, exit word */
 	reinterpret_cast<volatile uint32_t*>(m_rdone)[0] = 0u;
 	reinterpret_cast<volatile uint32_t*>(m_rdone)[1] = 0u;
@@ -1091,6 +1099,7 @@ Simulation::launchResident(uint32_t seq)
 	/* the launch gathers every cycle it updates */
 	m_pendingGather = false;
 	m_resident = true;
+	return seq;
 }
 
 void
@@ -1167,7 +1176,9 @@ Simulation::stepResident(const unsigned* fstim, size_t nf, const unsigned* inidx
 	bool done = false;
 	if(m_resident && m_turnWanted->load() == 0) {
 		std::lock_guard<std::mutex> guard(m_stayLock);
-		if(m_resident) {
+		if(m_resident && m_rseq >= RESIDENT_LAST - 1) {
+			endLaunch();   /* its last number */
+		} else if(m_resident) {
 			const uint32_t seq = ++m_rseq;
 			postCommand(seq, RESIDENT_STEP);
 			/* when the launch ended before the command: in a new one */
@@ -1181,8 +1192,7 @@ Simulation::stepResident(const unsigned* fstim, size_t nf, const unsigned* inidx
 			uint32_t seq = 0;
 			stayed = DeviceTurn::tryStay(m_device, this, [&] {
 				std::lock_guard<std::mutex> guard(m_stayLock);
-				seq = ++m_rseq;
-				launchResident(seq);
+				seq = launchResident();
 			});
 			if(stayed) {
 				std::lock_guard<std::mutex> guard(m_stayLock);

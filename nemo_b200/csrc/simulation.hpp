@@ -367,7 +367,7 @@ private:
 	bool stepResident(const unsigned* fstim, size_t nf, const unsigned* inidx, const float* icur, size_t ni);
 	bool mapInline(const unsigned* fstim, size_t nf, const unsigned* inidx, const float* icur, size_t ni);
 	bool fitsCommand() const { return 3u + m_inline.nf + 2u * m_inline.ni <= 3u * RESIDENT_CHUNKS; }
-	void launchResident(uint32_t seq);
+	uint32_t launchResident();
 	bool awaitCommand(uint32_t seq);
 	void endLaunch();
 	void endStay() noexcept override;
