@@ -19,23 +19,26 @@ ORACLE = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))
                       "libnemo_oracle.so")
 
 
-def _library(path, last):
+@pytest.fixture(scope="module")
+def numbers_lib(tmp_path_factory):
     b.build()
+    path = tmp_path_factory.mktemp("numbers")
     objs = [os.path.join(b.BUILD, f) for f in sorted(os.listdir(b.BUILD))
             if f.endswith(".o") and f != "simulation.cpp.o"]
-    obj = str(path / "simulation.o")
-    subprocess.check_call([b.CXX] + b.CXX_FLAGS + ["-DNEMO_B200_RESIDENT_LAST=%du" % last, "-c",
+    obj, lib = str(path / "simulation.o"), str(path / "libnemo_b200_numbers.so")
+    subprocess.check_call([b.CXX] + b.CXX_FLAGS + ["-DNEMO_B200_RESIDENT_LAST=40u", "-c",
                                                   os.path.join(b.CSRC, "simulation.cpp"), "-o", obj])
-    lib = str(path / "libnemo_b200_numbers.so")
     subprocess.check_call([b.CXX, obj] + objs + b.LINK + ["-o", lib])
-    return Library(lib)
+    lib = Library(lib)
+    lib.add_plugin_path(os.path.join(b.HERE, "plugins"))
+    return lib
 
 
 @pytest.mark.parametrize("n,m,stdp", [(900, 80, True), (5200, 60, False)])
-def test_numbers_start_again(tmp_path, n, m, stdp):
+def test_numbers_start_again(numbers_lib, n, m, stdp):
     spec = netgen.izhikevich_random(n, m, dmax=12, seed=n, stdp=stdp)
     sims = []
-    for lib in (_library(tmp_path, 40), Library(ORACLE)):
+    for lib in (numbers_lib, Library(ORACLE)):
         net = Network(lib)
         for p in spec.populations:
             net.add_neuron(net.add_neuron_type(p.type_name), p.idx, *p.args)
