@@ -319,19 +319,23 @@ Simulation::construct(const Network& net, const Configuration& conf, const Shard
 	}
 
 	/* update cost per owned warp: an HH warp (999 substeps of six exponentials
-	 * over eight lanes per neuron) counts 3 times another model's, so that
-	 * HH warps spread over more blocks while no block owns more warps than it
-	 * has update warps in a mixed network of a few HH neurons per ten others
-	 * (1,250 HH warps beside 1,407 others: at most 12 a block, three a
-	 * scheduler; with 2.5 times some blocks own 13 and a scheduler has four,
-	 * 716 clocks a substep against 587) */
+	 * over eight lanes per neuron) counts 3.5 times another model's. Its time
+	 * is a step function of the HH warps a scheduler has (430, 492, 587 and 716
+	 * clocks a substep with one to four), the others' rises with every warp of
+	 * a block; 3.5 is the best or within 1% of it over most of the range, us a
+	 * cycle of H HH neurons beside 45,000 others, weights 2.5 / 3 / 3.5 / 4 / 5:
+	 * H = 400: 493 / 475 / 470 / 477 / 477, 2,000: 507 / 512 / 506 / 517 / 508,
+	 * 3,000: 548 / 551 / 515 / 522 / 516, 3,500: 561 / 557 / 550 / 550 / 520,
+	 * 5,000: 615 / 570 / 566 / 567 / 569, 8,000: 698 / 696 / 692 / 639 / 635;
+	 * beside 9,000 others, 2,000: 456 / 446 / 440 / 440 / 439, 4,000: 483 / 479 /
+	 * 478 / 482 / 493 */
 	std::vector<uint32_t> warpCost(m_shard.warpHi - warpLo, 2u);
 	bool hh = false;
 	for(const Group& g : m_groups) {
 		if(g.type.kind != MODEL_HH) continue;
 		hh = true;
 		const uint32_t w0 = g.devBase / 32, w1 = uint32_t((uint64_t(g.devBase) + (uint64_t(g.count) << g.shift) + 31) / 32);
-		for(uint32_t w = std::max(w0, warpLo); w < std::min(w1, m_shard.warpHi); ++w) warpCost[w - warpLo] = 6u;
+		for(uint32_t w = std::max(w0, warpLo); w < std::min(w1, m_shard.warpHi); ++w) warpCost[w - warpLo] = 7u;
 	}
 	std::vector<uint32_t> ownStart;
 	uint32_t ownWarps = 0;
