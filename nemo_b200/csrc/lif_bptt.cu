@@ -513,6 +513,12 @@ static int rowWidth(int B) { return B <= 8 ? 8 : (B <= 16 ? 16 : 32); }
 
 const int ADJ_THREADS = 1024;
 const int ADJ_WARPS = ADJ_THREADS / 32;
+/* At least 8 parts also where fewer would hold the rows: a part's rows are
+ * read from L2 by every group each step, so few parts mean many rows a block;
+ * many parts mean sums to add. us a step with at least 2 / 4 / 8 / 16 parts:
+ * 300 neurons of 8 trials 4.4 / 4.7 / 4.6 / 5.2, 1,000 of 32 7.5 / 6.1 / 5.4 /
+ * 6.6, 2,000 of 32 10.4 / 7.7 / 7.5 / 9.0, 3,000 of 16 8.9 / 7.5 / 8.5 / 8.8,
+ * 5,000 of 32 14.0 / 14.0 / 12.2 / 12.5 */
 const int ADJ_MIN_PARTS = 8, ADJ_MAX_PARTS = 32;
 /* sources of a group (their places in a block's shared memory) */
 const size_t ADJ_SOURCES = 8192;
@@ -695,8 +701,8 @@ adjointRings(int tw)
 }
 
 /* Parts of the neurons: 8, or as many as it takes for a part's rows (and the
- * row of zeros) to fit a block beside its sources and rings; 0 past 32 parts
- * (40,000 neurons of 32 trials) */
+ * row of zeros) to fit a block beside its sources and rings (from 10,233
+ * neurons of 32 trials, 20,473 of 16 and 32,761 of 8 on); 0 past 32 parts */
 static int
 adjointParts(int N, int tw)
 {
@@ -1215,9 +1221,10 @@ struct AdjointPlan {
 	int groups = 0, partRows = 0, perGroup = 0;
 };
 
-/* The adjoint in one launch a segment, unless its rows ask for more parts than
- * there are (adjointParts): a group for every 64 sources, as many as run at
- * once. */
+/* The adjoint in one launch a segment: a group for every 64 sources, as many
+ * as run at once. Step by step where a group would have more sources than a
+ * block has places for, since many parts leave few groups: past 37,091 neurons
+ * of 32 trials (30 parts, four groups), 53,739 of 16, 65,520 of 8 on 148 SMs. */
 static AdjointPlan
 planAdjoint(const Net& n)
 {
@@ -1256,7 +1263,7 @@ struct ForwardPlan {
 };
 
 /* The forward in one launch, unless the spike words and v of a block do not
- * fit its shared memory (past 45,000 neurons): eight neurons a block at least,
+ * fit its shared memory (past 46,400 to 46,900 neurons, by the channels): eight neurons a block at least,
  * a warp a neuron, a large network's neurons two to four a warp at once. */
 static ForwardPlan
 planForward(const Net& n)

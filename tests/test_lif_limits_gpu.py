@@ -1,6 +1,7 @@
-"""The differentiable form past its kernels' shared memory: the one-launch pass
-against the captured one, which runs launch by launch and keeps nothing in
-shared memory. Spikes and counts are equal; gradients to rounding."""
+"""The differentiable form past its kernels' shared memory, and at the sizes
+where a direction goes back to a launch per step: against the captured pass,
+which runs launch by launch and keeps nothing in shared memory. Spikes and
+counts are equal; gradients to rounding."""
 
 import numpy as np
 import pytest
@@ -67,3 +68,17 @@ def test_entries_through_the_ring(dense, trials):
     # than a block has, at rows of 8, 16 and 32 trials; several passes, as the
     # ring is used anew every step
     _check(_problem(dense, 40, trials, seed=trials), passes=4)
+
+
+@pytest.mark.parametrize("n,n_rec,trials", [
+    (5000, 4_100_000, 9),    # 27,900 synapses a block, more than its room; two neurons a warp
+    (11000, 33_000, 32),     # nine parts of 32-trial rows (from 10,233 neurons on)
+    (20000, 60_000, 32),     # sixteen parts; more rows to finish than a block has threads
+    (37091, 80_000, 32),     # the largest network of 32 trials in one launch
+    (37092, 80_000, 32),     # the backward step by step
+    (48000, 90_000, 8),      # the forward step by step, the backward in 12 parts of 8-trial rows
+    (65600, 90_000, 5),      # both step by step
+])
+def test_sizes_at_the_limits(n, n_rec, trials):
+    net = _net(n, 20, n_rec, n, checkpoint=15, seed=n)
+    _check(_problem(net, 40, trials, seed=trials))
